@@ -95,22 +95,34 @@ def _normal(gen, rows, k, sigma, dtype):
     return x.normal_(0.0, sigma, generator=gen).to(dtype)
 
 
+def _is_mx(case):
+    return case["op"] == "mx_linear" or case.get("format") == "mx"
+
+
+def _product_inputs(case, gen):
+    """The weights [N, K] and activations [M, K] of a product before they are quantised."""
+    m, n, k = case["m"], case["n"], case["k"]
+    square = case["op"] == "gemm" and m == n == k                 # the benchmark's square products are N(0,1) on both sides
+    b = _normal(gen, n, k, 1.0 if square else 0.02, torch.bfloat16)
+    return b, _normal(gen, m, k, 1.0, torch.bfloat16 if case["op"] == "gemm" else DTYPES[case["x"]])
+
+
 def _prepare_product(case, gen):
     op, m, n, k = case["op"], case["m"], case["n"], case["k"]
-    mx = op == "mx_linear" or case.get("format") == "mx"
+    mx = _is_mx(case)
     pack = g.quantize_mx if mx else g.quantize
-    square = op == "gemm" and m == n == k                         # the benchmark's square products are N(0,1) on both sides
-    b, sfb = pack(_normal(gen, n, k, 1.0 if square else 0.02, torch.bfloat16))
+    b, x = _product_inputs(case, gen)
+    b, sfb = pack(b)
     if op == "mx_linear":
-        return {"op": op, "b": b, "sfb": sfb, "x": _normal(gen, m, k, 1.0, DTYPES[case["x"]]), "out": case["out"]}
+        return {"op": op, "b": b, "sfb": sfb, "x": x, "out": case["out"]}
     state = {"op": op}
     if op == "linear":
         # the plan's own A and scales: `linear` quantises into them
         a = torch.empty((m, k // 2), dtype=torch.uint8, device="cuda")
         sfa = torch.empty(scale_rows(m) * k // 16, dtype=torch.uint8, device="cuda")
-        state["x"] = _normal(gen, m, k, 1.0, DTYPES[case["x"]])
+        state["x"] = x
     else:
-        a, sfa = pack(_normal(gen, m, k, 1.0, torch.bfloat16))
+        a, sfa = pack(x)
         state["c"] = torch.empty((m, n), dtype=DTYPES[case["out"]], device="cuda")
     state["plan"] = g.Nvfp4Gemm(a, b, sfa, sfb, mx=mx)
     if case["out"] == "bf16":
@@ -118,21 +130,26 @@ def _prepare_product(case, gen):
     return state
 
 
-def _prepare_moe(case, gen):
+def _moe_inputs(case, gen):
     t, h, i, e, topk = (case[key] for key in ("tokens", "hidden", "inter", "experts", "topk"))
     w1 = torch.empty((e, 2 * i, h), dtype=torch.bfloat16, device="cuda").normal_(0.0, 0.02, generator=gen)
     w2 = torch.empty((e, h, i), dtype=torch.bfloat16, device="cuda").normal_(0.0, 0.02, generator=gen)
-    # a layer is sized for the largest batch it may see
-    layer = g.Nvfp4MoE(w1, w2, e, topk, clamp=10.0, max_tokens=256 if case["graph"] else 4096)
-    del w1, w2
     x = _normal(gen, t, h, 1.0, torch.bfloat16)
     logits = torch.randn((t, e), generator=gen, device="cuda")
     if case["skew"]:
         logits += case["skew"] * torch.randn((1, e), generator=gen, device="cuda")     # experts of unequal popularity
     ids, weights = g.route(logits, topk)
+    return w1, w2, x, ids, weights
+
+
+def _prepare_moe(case, gen):
+    w1, w2, x, ids, weights = _moe_inputs(case, gen)
+    # a layer is sized for the largest batch it may see
+    layer = g.Nvfp4MoE(w1, w2, case["experts"], case["topk"], clamp=10.0, max_tokens=256 if case["graph"] else 4096)
+    del w1, w2
     state = {"op": "moe", "layer": layer, "x": x, "ids": ids, "weights": weights}
     if case["graph"]:
-        state["captured"] = layer.capture(t)
+        state["captured"] = layer.capture(case["tokens"])
     return state
 
 
@@ -207,3 +224,58 @@ def tolerance(case):
     # the same in every order, and equal to the 64-bit product rounded once; what is allowed for is the last place of
     # the output type in a few values.
     return {"rel": 1e-4, "max": 1e-3} if case["out"] == "f16" else {"rel": 8e-4, "max": 8e-3}
+
+
+# ---- the same results in 64 bits, in plain torch ----------------------------------------------------------------
+
+
+def _e2m1(q):
+    """Quotients -> the nearest E2M1 values (ties to the even code), signs kept, in 64 bits."""
+    mag = q.abs().double()
+    level = torch.tensor([0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0], dtype=torch.float64, device=q.device)
+    mid = torch.tensor([0.25, 0.75, 1.25, 1.75, 2.5, 3.5, 5.0], dtype=torch.float64, device=q.device)
+    code = torch.bucketize(mag, mid)                              # midpoints below the magnitude
+    on = mag == mid[code.clamp(max=6)]
+    code += on & (code % 2 == 1)
+    return torch.where(q < 0, -level[code], level[code])
+
+
+def _rounded(x, mx):
+    """x [rows, K] -> the values its NVFP4 (or MXFP4) form stands for, in 64 bits; by row blocks, to bound the memory."""
+    out = torch.empty(x.shape, dtype=torch.float64, device=x.device)
+    step = max(1, (1 << 25) // x.shape[1])
+    for r in range(0, x.shape[0], step):
+        part = x[r:r + step].float()
+        blocks = part.reshape(part.shape[0], -1, 32 if mx else 16)
+        amax = blocks.abs().amax(-1, keepdim=True)
+        if mx:
+            scale = torch.exp2((torch.frexp(amax).exponent - 3).double())
+        else:
+            scale = (amax / 6.0).clamp(2.0 ** -9, 448.0).to(torch.float8_e4m3fn).double()
+        out[r:r + step] = (_e2m1(blocks / scale.float()) * scale).reshape(part.shape)
+    return out
+
+
+def _exact_moe(case, gen):
+    w1, w2, x, ids, weights = _moe_inputs(case, gen)
+    inter = case["inter"]
+    x = _rounded(x, False)
+    slots = torch.zeros((*ids.shape, case["hidden"]), dtype=torch.float64, device="cuda")
+    for e in ids.unique().tolist():
+        token, slot = torch.nonzero(ids == e, as_tuple=True)
+        gate_up = (x[token] @ _rounded(w1[e], False).T).bfloat16().double()            # the layer's own rounding points
+        gate, up = gate_up[:, :inter].clamp(max=10.0), gate_up[:, inter:].clamp(-10.0, 10.0)
+        act = (gate * torch.sigmoid(gate) * up * weights[token, slot].double()[:, None]).bfloat16()
+        slots[token, slot] = (_rounded(act, False) @ _rounded(w2[e], False).T).bfloat16().double()
+    return slots.sum(1)
+
+
+def exact(case, seed):
+    gen = torch.Generator(device="cuda").manual_seed(int(seed))
+    if case["op"] == "quantize":
+        return None                                               # bytes: compared as they are
+    if case["op"] == "moe":
+        return _exact_moe(case, gen)
+    b, x = _product_inputs(case, gen)
+    mx = _is_mx(case)
+    return _rounded(x, mx) @ _rounded(b, mx).T
