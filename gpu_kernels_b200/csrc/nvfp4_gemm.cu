@@ -532,11 +532,14 @@ struct Roles {
                     tc_fence_after_sync();
                 }
                 if (elect_one()) {
-                    #pragma unroll
-                    for (int j = 0; j < STAGE_K / MMA_K; ++j) {
-                        if (!handover) copies(j);
-                        mma(j);
+                    // All copies of the step before its first MMA: a copy behind an MMA waits for it, so alternating
+                    // the two drains the pipe four times a step instead of once.
+                    if (!handover) {
+                        #pragma unroll
+                        for (int j = 0; j < STAGE_K / MMA_K; ++j) copies(j);
                     }
+                    #pragma unroll
+                    for (int j = 0; j < STAGE_K / MMA_K; ++j) mma(j);
                     mma_commit<CG>(empty);                      // stage reusable once these MMAs retire
                     if (ks == seg.k1 - 1) mma_commit<CG>(bar(&ctrl->acc_full));
                 }
