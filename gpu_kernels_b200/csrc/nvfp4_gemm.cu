@@ -77,14 +77,14 @@ enum Epi : int {
 template <int CG, int UN, int EPI, bool MX = false>
 struct Config {
     static_assert(CG == 1 || CG == 2, "cta group");
-    static_assert(UN == 128 || UN == 256, "tile width");
+    static_assert(UN == 64 || UN == 128 || UN == 256, "tile width");
     static constexpr int TILE_M = BLOCK_M * CG;
     static constexpr int B_ROWS = UN / CG;                       // B rows staged by each CTA
     static constexpr int A_BYTES = BLOCK_M * ROW_BYTES;
     static constexpr int B_BYTES = B_ROWS * ROW_BYTES;
     static constexpr int SF_SLOTS = MX ? STAGE_K / 128 : STAGE_K / MMA_K;      // scale atoms per 128 rows and ring stage
     static constexpr int SFA_BYTES = SF_SLOTS * SF_ATOM_BYTES;
-    static constexpr int SFB_BLOCKS = UN / 128;                  // 128-row scale blocks across the tile width
+    static constexpr int SFB_BLOCKS = (UN + 127) / 128;          // 128-row scale blocks the tile's columns lie in
     static constexpr int SFB_BLOCK_BYTES = SF_SLOTS * SF_ATOM_BYTES;
     static constexpr int SFB_BYTES = SFB_BLOCKS * SFB_BLOCK_BYTES;
     static constexpr int OFF_B = A_BYTES;
@@ -117,7 +117,7 @@ struct Config {
     static constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + EPI_BYTES + CTRL_BYTES;
     // Tensor Memory columns: scale columns for the four MMAs of a stage at the top,
     // two accumulators below them (overlapping when they cannot both fit).
-    static constexpr int SF_COLS_PER_MMA = 4 + UN / 32;          // columns of one atom of SFA and the tile's atoms of SFB
+    static constexpr int SF_COLS_PER_MMA = 4 + 4 * SFB_BLOCKS;   // columns of one atom of SFA and the tile's atoms of SFB
     static constexpr int SF_COLS = SF_SLOTS * SF_COLS_PER_MMA;
     static constexpr int SF_BASE = TMEM_COLS - SF_COLS;
     static constexpr int ACC_STRIDE = (2 * UN <= SF_BASE) ? UN : SF_BASE - UN;
@@ -180,7 +180,8 @@ struct GemmArgs {
     void* const* slots;             // device array of `world` buffer addresses
     int world;
     int slot_rows;
-    // Tile t walks K starting at step (t * k_skew) % ksteps and wraps: the CTAs then do not all ask HBM for
+    // A tile walks K starting at step (place * k_skew) % ksteps and wraps, where place counts the 256-wide blocks of
+    // C (dense) or is the tile's index (grouped and ragged): the CTAs then do not all ask HBM for
     // the same 128-byte column of their rows at the same time. 0 = every tile starts at K = 0.
     int k_skew;
     // EPI_SPLIT_K (dense mode, shapes with far fewer tiles than SMs): unit u works on K steps
@@ -220,6 +221,10 @@ struct GemmArgs {
     // fetched in 64-row boxes; a tile's scale atoms are the two 128-row blocks its columns lie in, and the MMA
     // reads them from the column (n0 % 128) / 32 on.
     int ragged_base, ragged_extra;
+    // Rows of A's box (CG = 1): 128, or M rounded up to 8 rows when M < 128. The rows of the stage a smaller box does
+    // not reach keep whatever bytes they hold: every E2M1 code is finite, a row of the product depends on its own row
+    // of A alone, and rows >= M are never stored.
+    int a_box_rows;
 };
 
 // First column and width of tile tn of a ragged row of tiles.
@@ -349,6 +354,30 @@ struct Roles {
             int sfb_block = (b_base + tn * UN) / 128;
             int b_boxes = 1;                                    // 64-row boxes of B per stage (ragged tiles only)
             uint32_t stage_bytes = Cfg::STAGE_BYTES;
+            // Boxes that lie wholly beyond A or B (the second half of a last, partial 256-wide tile) are not
+            // requested: what they stand for is not stored, and a box of rows the tensor does not have takes the
+            // copy unit longer than one it has to fetch (about 6 cycles a row).
+            bool b_live = true;
+            int sfb_live = Cfg::SFB_BLOCKS;
+            if constexpr (EPI == EPI_DIRECT_EDGE) {
+                if (!g.block_expert) {
+                    const int blocks = (g.N + 127) / 128;
+                    b_live = b_row < g.N;
+                    sfb_live = min(Cfg::SFB_BLOCKS, blocks - sfb_block);
+                    const int first_b = tn * UN;
+                    const int live_b = CG == 2 ? 1 + int(first_b + Cfg::B_ROWS < g.N) : 1;       // boxes of the pair
+                    stage_bytes = uint32_t(g.a_box_rows * ROW_BYTES + Cfg::SFA_BYTES + sfb_live * Cfg::SFB_BLOCK_BYTES) * CG +
+                                  uint32_t(live_b * Cfg::B_BYTES);
+                    const int live_a = CG == 2 ? 1 + int(tm * Cfg::TILE_M + BLOCK_M < g.M) : 1;
+                    if (live_a < CG) stage_bytes -= uint32_t(Cfg::A_BYTES + Cfg::SFA_BYTES);
+                } else {
+                    stage_bytes = CG * Cfg::STAGE_BYTES;
+                }
+            } else {
+                stage_bytes = CG * Cfg::STAGE_BYTES;
+            }
+            const bool a_live = EPI != EPI_DIRECT_EDGE || CG == 1 || a_row < g.M;
+            const bool whole = EPI != EPI_DIRECT_EDGE || (a_live && b_live && sfb_live == Cfg::SFB_BLOCKS);
             if constexpr (Cfg::RAGGED) {
                 int n0, width;
                 ragged_span(g, tn, n0, width);
@@ -358,7 +387,10 @@ struct Roles {
                 stage_bytes = Cfg::A_BYTES + uint32_t(width) * ROW_BYTES + Cfg::SFA_BYTES + Cfg::SFB_BYTES;
             }
             // whole tiles may start anywhere in K and wrap; slices of a tile are walked in order
-            const int k_first = (g.k_skew && g.split_k <= 1) ? int((t * uint32_t(g.k_skew)) % uint32_t(ksteps)) : 0;
+            // (see GemmArgs::k_skew); a dense C's walk depends on the 256 x 256 block of C, not on the tile, so that
+            // its sums are taken in the same order whatever the tiles are
+            const uint32_t place = g.block_expert || Cfg::RAGGED ? t : uint32_t(tn * UN / 256 + 5 * (tm * Cfg::TILE_M / 256));
+            const int k_first = (g.k_skew && g.split_k <= 1) ? int((place * uint32_t(g.k_skew)) % uint32_t(ksteps)) : 0;
             for (int step = seg.k0; step < seg.k1; ++step) {
                 const int ks = step + k_first < ksteps ? step + k_first : step + k_first - ksteps;
                 const long long w0 = now();
@@ -371,7 +403,7 @@ struct Roles {
                 // The first ring fill of a launch whose B is static goes out in two halves: B and its scales at
                 // once, A and its scales after the grid in front of this launch has finished (see below).
                 const bool split_issue = early_b && issued < Cfg::STAGES;
-                if (split_issue) held[issued] = {ks, a_row, sfa_block};
+                if (split_issue) held[issued] = {ks, a_live ? a_row : -1, sfa_block};
                 if constexpr (CG == 1) {
                     if (elect_one()) {
                         mbar_arrive_expect_tx(own_full, stage_bytes);
@@ -387,23 +419,29 @@ struct Roles {
                         }
                         #pragma unroll
                         for (int b = 0; b < Cfg::SFB_BLOCKS; ++b)
-                            tma_load_3d(base + Cfg::OFF_SFB + b * Cfg::SFB_BLOCK_BYTES, tmSFB, 0, ks * (Cfg::SF_SLOTS * 4),
-                                        sfb_block + b, own_full);
+                            if (whole || b < sfb_live)
+                                tma_load_3d(base + Cfg::OFF_SFB + b * Cfg::SFB_BLOCK_BYTES, tmSFB, 0, ks * (Cfg::SF_SLOTS * 4),
+                                            sfb_block + b, own_full);
                     }
                 } else {
                     // Both CTAs of the pair report their bytes to the leader's barrier.
                     const uint32_t full = map_to_cta(own_full, 0);
-                    if (elect_one()) {
-                        if (rank == 0) mbar_arrive_expect_tx(own_full, 2 * Cfg::STAGE_BYTES);
-                        if (!split_issue) {
+                    auto request = [&](bool a, bool b_rows, int sfb_blocks) {
+                        if (rank == 0) mbar_arrive_expect_tx(own_full, stage_bytes);
+                        if (a) {
                             tma_load_2d_pair(base, tmA, ks * ROW_BYTES, a_row, full);
                             tma_load_3d_pair(base + Cfg::OFF_SFA, tmSFA, 0, ks * (Cfg::SF_SLOTS * 4), sfa_block, full);
                         }
-                        tma_load_2d_pair(base + Cfg::OFF_B, tmB, ks * ROW_BYTES, b_row, full);
+                        if (b_rows) tma_load_2d_pair(base + Cfg::OFF_B, tmB, ks * ROW_BYTES, b_row, full);
                         #pragma unroll
                         for (int b = 0; b < Cfg::SFB_BLOCKS; ++b)
-                            tma_load_3d_pair(base + Cfg::OFF_SFB + b * Cfg::SFB_BLOCK_BYTES, tmSFB, 0, ks * (Cfg::SF_SLOTS * 4),
-                                             sfb_block + b, full);
+                            if (b < sfb_blocks)
+                                tma_load_3d_pair(base + Cfg::OFF_SFB + b * Cfg::SFB_BLOCK_BYTES, tmSFB, 0, ks * (Cfg::SF_SLOTS * 4),
+                                                 sfb_block + b, full);
+                    };
+                    if (elect_one()) {
+                        if (whole) request(!split_issue, true, Cfg::SFB_BLOCKS);
+                        else request(!split_issue && a_live, b_live, sfb_live);
                     }
                 }
                 ++issued;
@@ -431,7 +469,7 @@ struct Roles {
                 if constexpr (CG == 1) {
                     tma_load_2d(base, tmA, held[i].ks * ROW_BYTES, held[i].a_row, own_full);
                     tma_load_3d(base + Cfg::OFF_SFA, tmSFA, 0, held[i].ks * (Cfg::SF_SLOTS * 4), held[i].sfa_block, own_full);
-                } else {
+                } else if (held[i].a_row >= 0) {
                     const uint32_t full = map_to_cta(own_full, 0);
                     tma_load_2d_pair(base, tmA, held[i].ks * ROW_BYTES, held[i].a_row, full);
                     tma_load_3d_pair(base + Cfg::OFF_SFA, tmSFA, 0, held[i].ks * (Cfg::SF_SLOTS * 4), held[i].sfa_block, full);
@@ -473,6 +511,10 @@ struct Roles {
                 ragged_span(g, tn, n0, width);
                 idesc = (1u << 7) | (1u << 10) | (uint32_t(width >> 3) << 17) | (uint32_t(Cfg::TILE_M >> 4) << 24);
                 sfb_shift = uint32_t(n0 % 128) / 32u;           // the tile's first row inside its first scale atom
+            } else if constexpr (UN % 128 != 0) {
+                int tm, tn, b_base;
+                tile_coords(int(seg.tile), g, tm, tn, b_base);
+                sfb_shift = uint32_t((tn * UN) % 128) / 32u;
             }
             unsigned long long* tr = nullptr;
             if (PROF && unit == 0 && lane == 0 && iter > 0 && iter <= TR_TILES)
@@ -1111,6 +1153,7 @@ int max_units(int device) {
 }
 
 int fit_units(int device, int cta_group, int tile_n) {
+    // single CTAs: one per SM, whatever the width
     return cta_group == 2 ? max_units<2, 256>(device) : tile_n == 256 ? max_units<1, 256>(device) : max_units<1, 128>(device);
 }
 
@@ -1126,6 +1169,62 @@ uint32_t* status_base(int device) {
 uint32_t* status_slot(int device, int slot) { return status_base(device) + size_t(slot) * 4; }
 
 std::atomic<unsigned> g_next_slot{0};
+
+// Rows of A's box: a tensor of fewer than 128 rows is fetched without the rows it does not have (see
+// GemmArgs::a_box_rows). With whole boxes 8 x 8192 x 8192 on 128-wide tiles took 20.3 us, with 8-row boxes 14.8 us.
+int a_box_rows(int M) { return M < BLOCK_M ? (M + 7) / 8 * 8 : BLOCK_M; }
+
+// About sqrt(units) tile rows per band keeps the A and B panels of the tiles in flight balanced.
+// Measured at 16384^3 (64 x 64 tiles, operands beyond L2): bands of 16 beat 8 by 1.3 %, 32 and 4 lose 10 %;
+// at 8192^3 (everything L2-resident) the band height does not matter.
+int band_rows(int units, int tiles_m) {
+    int gm = 1;
+    while ((gm + 1) * (gm + 1) <= units) ++gm;
+    if (tiles_m >= 48) gm = std::max(gm, 16);
+    return std::max(1, std::min(gm, tiles_m));
+}
+
+// The tiles of a plain launch. The plan's own (cta_group, tile_n) are whole tiles of the padded shape, which the
+// other routes need; for a plain launch two cases are faster on other tiles, with the masked epilogue:
+//   * few tiles: a tile's K loop is bound by the instructions that feed it, about the same number per step for 64
+//     columns as for 256, so narrower tiles finish sooner as long as every one has an SM of its own;
+//   * M or N an odd multiple of 128: the plan falls back to single-CTA tiles, although CTA pairs with a half-empty
+//     last tile move half the bytes per FLOP.
+// Time estimate in ns: launch and first data, the exposed epilogue of the last tile, then a cost per ring step and
+// wave; fitted to M = 8..1024, N = 1536..28672, K = 2048..8192 within 10 %. At least as long as the weights need
+// from HBM. Measured (us, the plan's own tiles / these): 8 x 8192 x 8192 16.9 / 12.9, 128 x 4096 x 4096 11.5 / 8.0,
+// 512 x 2048 x 4096 10.0 / 8.2, 8 x 14336 x 4096 11.4 / 9.4, 4096 x 4224 x 4096 49.2 / 39.4, 4100 x 8320 x 4096
+// 103.6 / 83.0; where these would lose: 128 x 28672 x 8192 on 128-wide tiles 27.3 / 29.6.
+struct PlainTile { int cta_group, tile_n; float step_ns, tail_ns; };
+constexpr PlainTile PLAIN_TILES[] = {{2, 256, 380.0f, 1000.0f}, {1, 256, 430.0f, 1000.0f}, {1, 128, 320.0f, 500.0f}, {1, 64, 290.0f, 300.0f}};
+
+void choose_plain_tiles(gpu_kernels::Nvfp4Params& p, const uint8_t* B, int forced) {
+    const int steps = (p.K + STAGE_K - 1) / STAGE_K;
+    const float hbm_ns = float(p.N) * float(p.K) * (p.mx ? 0.53125f : 0.5625f) / 6500.0f;
+    auto tiles = [&](const PlainTile& t) { return ((p.M + 128 * t.cta_group - 1) / (128 * t.cta_group)) * ((p.N + t.tile_n - 1) / t.tile_n); };
+    auto estimate = [&](const PlainTile& t, int waves) { return 3000.0f + t.tail_ns + std::max(hbm_ns, float(waves) * float(steps) * t.step_ns); };
+    const PlainTile* best = nullptr;
+    float best_ns = 0.0f;
+    for (const PlainTile& t : PLAIN_TILES)
+        if (t.cta_group == p.cta_group && t.tile_n == p.tile_n)
+            best_ns = 0.95f * estimate(t, (tiles(t) + p.clusters - 1) / p.clusters);       // another tile has to gain 5 %
+    for (const PlainTile& t : PLAIN_TILES) {
+        if (t.cta_group == p.cta_group && t.tile_n == p.tile_n) continue;
+        const int fit = fit_units(p.device, t.cta_group, t.tile_n), n = tiles(t), waves = (n + fit - 1) / fit;
+        const bool wider = t.cta_group * t.tile_n > p.cta_group * p.tile_n;
+        if (wider ? steps < 4 : waves > 1) continue;         // narrow tiles only while each has an SM; a short K loop is all epilogue
+        const float ns = estimate(t, waves);
+        if (ns < best_ns) { best_ns = ns; best = &t; }
+    }
+    if (forced == 1064) best = &PLAIN_TILES[3];
+    if (!best) return;
+    const int tiles_m = (p.M + 128 * best->cta_group - 1) / (128 * best->cta_group);
+    p.plain_cta_group = best->cta_group;
+    p.plain_tile_n = best->tile_n;
+    p.plain_units = std::min(fit_units(p.device, best->cta_group, best->tile_n), tiles(*best));
+    p.plain_group_m = band_rows(p.plain_units, tiles_m);
+    p.plain_B = operand_map(B, p.N, p.K, best->tile_n / best->cta_group);
+}
 
 // Ragged tiling of a one-tile-row plan over `tiles` single-CTA tiles (see GemmArgs::ragged_base); tiles = 0
 // switches it off. Returns whether the plan now uses it: M = 128, single-CTA 256-column variant, the widths
@@ -1163,7 +1262,10 @@ void prepare_format(gpu_kernels::Nvfp4Params& p, const uint8_t* A, const uint8_t
     p.device = device;
     p.c_evict_first = env_int("NVFP4_B200_C_EVICT_FIRST", 1);
 
-    const int force = env_int("NVFP4_B200_VARIANT", 0);        // 0 auto, 2256 / 1256 / 1128 for experiments
+    int force = env_int("NVFP4_B200_VARIANT", 0);              // 0 auto, 2256 / 1256 / 1128 / 1064 for experiments
+    const bool own_tiles = force != 0 && force != 1064;        // 1064: the plan as usual, its plain launches on 64-wide tiles
+    const int plain = force;
+    if (!own_tiles) force = 0;
     // M and N need not be whole tiles: the scale arrays end in whole 128-row atoms whatever the row count (rows
     // the tensor does not have read as zeros through the tensor maps), and the variant is chosen for the sizes
     // rounded up to 128.
@@ -1178,19 +1280,14 @@ void prepare_format(gpu_kernels::Nvfp4Params& p, const uint8_t* A, const uint8_t
     // 1717 / 1753 us, 8192x4096x2048 36.3 / 38.6 us. Single-CTA tiles have no staged route.
     p.direct_store = p.cta_group == 1 ? 1 : env_int("NVFP4_B200_DIRECT_STORE", 1);
     const int box_b = p.tile_n / p.cta_group;
-    p.A = operand_map(A, M, K, BLOCK_M);
+    p.A = operand_map(A, M, K, a_box_rows(M));
     p.B = operand_map(B, N, K, box_b);
     p.SFA = scale_map(SFA, M, K, mx ? 128 : 64);
     p.SFB = scale_map(SFB, N, K, mx ? 128 : 64);
     const int tiles = (Mp / (128 * p.cta_group)) * (Np / p.tile_n);
     p.clusters = std::min(fit_units(device, p.cta_group, p.tile_n), tiles);
-    // About sqrt(units) tile rows per band keeps the A and B panels of the tiles in flight balanced.
-    int gm = 1;
-    while ((gm + 1) * (gm + 1) <= p.clusters) ++gm;
-    // Measured at 16384^3 (64 x 64 tiles, operands beyond L2): bands of 16 beat 8 by 1.3 %, 32 and 4 lose 10 %;
-    // at 8192^3 (everything L2-resident) the band height does not matter.
-    if (Mp / (128 * p.cta_group) >= 48) gm = std::max(gm, 16);
-    p.group_m = std::max(1, std::min(env_int("NVFP4_B200_GROUP_M", gm), Mp / (128 * p.cta_group)));
+    const int tiles_m = Mp / (128 * p.cta_group);
+    p.group_m = std::max(1, std::min(env_int("NVFP4_B200_GROUP_M", band_rows(p.clusters, tiles_m)), tiles_m));
     // Measured: 128x28672x8192 30.2 -> 28.9 us, 8192^3 199.8 -> 199.0 us with the tiles' K walks de-phased.
     p.k_skew = env_int("NVFP4_B200_K_SKEW", 11);
     // One tile row whose 256-column tiles would leave SMs idle can deal its columns, in units of 64, to as many
@@ -1200,6 +1297,7 @@ void prepare_format(gpu_kernels::Nvfp4Params& p, const uint8_t* A, const uint8_t
     // launches: 28.5 against 24.7-26.1 us).
     if (!mx && env_int("NVFP4_B200_RAGGED", 0)) set_ragged_tiles(p, B, fit_units(device, 1, 256));
     p.pdl = env_int("NVFP4_B200_PDL", 1);
+    if (!own_tiles) choose_plain_tiles(p, B, plain);
     p.status_slot = 1 + int(g_next_slot.fetch_add(1, std::memory_order_relaxed) % unsigned(STATUS_SLOTS - 1));
     (void)status_base(device);
 }
@@ -1297,6 +1395,7 @@ GemmArgs dense_args(const gpu_kernels::Nvfp4Params& p, void* c, unsigned long lo
     g.c = c;
     g.ldc = p.N;
     g.c_rows_32 = rows_start_on_32(c, p.N);
+    g.a_box_rows = a_box_rows(p.M);
     g.k_skew = p.k_skew;
     g.split_k = p.split_k;
     if (p.split_k > 1) {
@@ -1361,11 +1460,30 @@ void launch_dense(const gpu_kernels::Nvfp4Params& p, const CUtensorMap& tmC, con
     }
 }
 
+// A plain launch on the tiles of choose_plain_tiles.
+template <int CG, int UN>
+void launch_plain(const gpu_kernels::Nvfp4Params& p, const CUtensorMap& tmC, const GemmArgs& dense, cudaStream_t stream) {
+    GemmArgs g = dense;
+    g.tiles_m = (p.M + 128 * CG - 1) / (128 * CG);
+    g.tiles_n = (p.N + UN - 1) / UN;
+    g.group_m = p.plain_group_m;
+    const bool pdl = p.pdl != 0;
+    if (p.mx) launch_instance<CG, UN, EPI_DIRECT_EDGE, false, true>(p.device, p.plain_units, p.A, p.plain_B, p.SFA, p.SFB, tmC, g, stream, pdl);
+    else launch_instance<CG, UN, EPI_DIRECT_EDGE>(p.device, p.plain_units, p.A, p.plain_B, p.SFA, p.SFB, tmC, g, stream, pdl);
+}
+
 void launch_with(const gpu_kernels::Nvfp4Params& p, void* C, cudaStream_t stream, unsigned long long* prof) {
     if (!C || (reinterpret_cast<uintptr_t>(C) & 15)) throw std::invalid_argument("nvfp4 gemm: C must be 16-byte aligned");
     if (prof && (p.split_k > 1 || p.gather_world)) throw std::invalid_argument("nvfp4 gemm profile: plain plans only");
     const CUtensorMap tmC = output_map(C, p.M, p.N, p.out_bf16 != 0);
     const GemmArgs g = dense_args(p, C, prof);
+    if (p.plain_tile_n && p.split_k <= 1 && !p.gather_world && !p.ragged_units && !p.route && p.direct_store && !prof) {
+        if (p.plain_cta_group == 2) launch_plain<2, 256>(p, tmC, g, stream);
+        else if (p.plain_tile_n == 256) launch_plain<1, 256>(p, tmC, g, stream);
+        else if (p.plain_tile_n == 128) launch_plain<1, 128>(p, tmC, g, stream);
+        else launch_plain<1, 64>(p, tmC, g, stream);
+        return;
+    }
     if (p.cta_group == 2) launch_dense<2, 256>(p, tmC, g, stream);
     else if (p.tile_n == 256) launch_dense<1, 256>(p, tmC, g, stream);
     else launch_dense<1, 128>(p, tmC, g, stream);

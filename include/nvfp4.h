@@ -65,6 +65,10 @@ struct Nvfp4Params {
     CUtensorMap B64;
     int ragged_base, ragged_extra, ragged_units;
     int mx;                         // 1: MXFP4 operands (one UE8M0 scale per 32 values), see mxfp4_prepare
+    // Tiles of a plain launch (no split-K, gather, ragged tiles, L2-side order, staged stores or profile) where
+    // another tile than cta_group x tile_n finishes the shape sooner; plain_tile_n = 0: the same tiles.
+    int plain_cta_group, plain_tile_n, plain_units, plain_group_m;
+    CUtensorMap plain_B;
 };
 
 struct Nvfp4Implementation {

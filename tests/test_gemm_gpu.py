@@ -429,6 +429,45 @@ def test_m_and_n_that_are_not_whole_tiles(g, m, n, k, variant):
     plan.close()
 
 
+# Plain launches on other tiles than the plan's own: 64-wide tiles forced (odd tiles start in the middle of a scale
+# atom; A boxes of fewer than 128 rows), and shapes where the rule takes narrow tiles for few columns, or CTA pairs
+# whose last tile has a half that lies wholly beyond N or M. (M, N, K, what the plan's own tiles are)
+PLAIN_TILE_SHAPES = [
+    (1, 8, 64, 1064), (7, 136, 320, 1064), (129, 72, 512, 1064), (128, 192, 1088, 1064), (300, 1000, 2304, 1064),
+    (8, 8192, 2048, 1256), (512, 2048, 2048, 2256), (121, 3000, 1024, 1256), (1000, 4224, 1280, 1128), (300, 8192, 1536, 1256),
+    (1100, 4360, 1088, 1128),
+]
+
+
+@pytest.mark.parametrize("m,n,k,variant", PLAIN_TILE_SHAPES)
+def test_plain_launch_on_other_tiles(g, m, n, k, variant):
+    pa, sa = g.quantize(random_operand(m, k, seed=m + n))
+    pb, sb = g.quantize(random_operand(n, k, seed=m + k, scale=0.05))
+    ua, ub = g.unpack_scales(sa, -(-m // 128) * 128, k), g.unpack_scales(sb, -(-n // 128) * 128, k)
+    ua[m:] = 0x7F                                            # NaN scales in the rows the tensors do not have
+    ub[n:] = 0x7F
+    sa2, sb2 = g.pack_scales(ua), g.pack_scales(ub)
+    if variant == 1064:
+        os.environ["NVFP4_B200_VARIANT"] = "1064"
+    try:
+        plan = g.Nvfp4Gemm(pa, pb, sa2, sb2)
+    finally:
+        os.environ.pop("NVFP4_B200_VARIANT", None)
+    info = plan.info()
+    assert variant == 1064 or info["cta_group"] * 1000 + info["tile_n"] == variant, info
+    whole = torch.full((m + 3, n), float("nan"), dtype=torch.float16, device="cuda")
+    whole[m:] = 77.0
+    out = plan.run(whole[:m])
+    plan.validate()
+    ref = g.dequantize(pa, sa) @ g.dequantize(pb, sb).T
+    assert_gemm_close(out, to_np(ref), f"plain tiles {m}x{n}x{k}")
+    assert bool((whole[m:] == 77.0).all()), "rows beyond M were written"
+    # the plan's own tiles take every sum in the same order: the same bits
+    own, _ = run_plan(g, pa, sa2, pb, sb2, variant=info["cta_group"] * 1000 + info["tile_n"])
+    assert torch.equal(out, own)
+    plan.close()
+
+
 def test_mxfp4_edge_shapes(g):
     for m, n, k in [(1, 264, 256), (100, 200, 512), (500, 1000, 384)]:
         a = random_operand(m, k, seed=m + k)
