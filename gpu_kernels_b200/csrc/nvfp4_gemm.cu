@@ -808,7 +808,7 @@ struct Roles {
                 } else if constexpr (EPI == EPI_ACT) {
                     const int inter = g.N / 2;
                     const int row = row0 + lane;
-                    const float w = __ldg(g.row_weight + row);
+                    const float w = row < row_limit ? __ldg(g.row_weight + row) : 0.0f;     // behind the real rows: whatever an earlier batch left
                     const int act_col = tn * (UN / 2) + chunk * (EPI_COLS / 2);        // first activation column of this chunk
                     uint2 codes[2];
                     uint32_t sb[2];

@@ -74,27 +74,41 @@ __global__ void route_count_kernel(const long long* __restrict__ ids, int routes
         if (local[e]) atomicAdd(&counts[e], local[e]);
 }
 
-// Exclusive prefix sum over n <= 4096 ints held in shared memory, by one CTA of 256 threads: each thread
-// scans a contiguous chunk serially, the chunk totals are scanned by one thread (<= 256 values).
-__device__ void block_exclusive_scan(int* data, int n, int* chunk_sums) {
-    const int per = (n + int(blockDim.x) - 1) / int(blockDim.x);
+constexpr int PLAN_THREADS = 1024;
+
+// Exclusive prefix sum over n <= 4096 ints held in shared memory, by one CTA of PLAN_THREADS threads: each thread
+// scans a contiguous chunk, the chunk totals are scanned across the lanes of a warp and then across the 32 warps (one
+// thread adding up 256 chunk totals took most of the kernel's 10 us). sums: 33 ints; sums[32] = the total.
+__device__ void block_exclusive_scan(int* data, int n, int* sums) {
+    const int per = (n + PLAN_THREADS - 1) / PLAN_THREADS, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int lo = min(int(threadIdx.x) * per, n), hi = min(lo + per, n);
     int acc = 0;
-    for (int i = lo; i < hi; ++i) { const int v = data[i]; data[i] = acc; acc += v; }
-    chunk_sums[threadIdx.x] = acc;
+    for (int i = lo; i < hi; ++i) acc += data[i];
+    auto inclusive = [&](int v) {
+        #pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int up = __shfl_up_sync(0xFFFFFFFFu, v, d);
+            if (lane >= d) v += up;
+        }
+        return v;
+    };
+    const int upto = inclusive(acc);
+    if (lane == 31) sums[warp] = upto;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int run = 0;
-        for (unsigned i = 0; i < blockDim.x; ++i) { const int v = chunk_sums[i]; chunk_sums[i] = run; run += v; }
-        chunk_sums[blockDim.x] = run;
+    if (warp == 0) {
+        const int v = sums[lane], w = inclusive(v);
+        __syncwarp();
+        sums[lane] = w - v;
+        if (lane == 31) sums[32] = w;
     }
     __syncthreads();
-    for (int i = lo; i < hi; ++i) data[i] += chunk_sums[threadIdx.x];
+    int run = sums[warp] + upto - acc;
+    for (int i = lo; i < hi; ++i) { const int v = data[i]; data[i] = run; run += v; }
     __syncthreads();
 }
 
-// counts[r * experts + ge]: routes rank r sends to global expert ge. One CTA of 256 threads; experts <= 4096.
-__global__ void plan_kernel(int* __restrict__ block_valid, int* counts, int world, int rank, int experts, int capacity_rows,
+// counts[r * experts + ge]: routes rank r sends to global expert ge. One CTA of PLAN_THREADS threads; experts <= 4096.
+__global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(int* __restrict__ block_valid, int* counts, int world, int rank, int experts, int capacity_rows,
                             int block_rows,
                             int* __restrict__ send_offset, int* __restrict__ seg_src_offset,
                             int* __restrict__ seg_pool_offset, int* __restrict__ block_expert,
@@ -106,7 +120,7 @@ __global__ void plan_kernel(int* __restrict__ block_valid, int* counts, int worl
     const int segments = world * local_experts;          // == experts
     int* scan = sh;                                       // [experts] scratch for the three scans
     int* pool_off = sh + experts;                         // [local_experts] padded start of each expert
-    int* chunk = pool_off + local_experts;                // [blockDim.x + 1]
+    int* chunk = pool_off + local_experts;                // [33]
     if (ids) {
         // One rank: nothing to exchange, so the histogram of the routes is taken right here (the counts row is
         // this kernel's own output) instead of by a zeroing memset and a counting kernel before it.
@@ -127,7 +141,7 @@ __global__ void plan_kernel(int* __restrict__ block_valid, int* counts, int worl
     __syncthreads();
     block_exclusive_scan(scan, experts, chunk);
     for (int ge = threadIdx.x; ge < experts; ge += blockDim.x) send_offset[ge] = scan[ge];
-    if (threadIdx.x == 0) send_offset[experts] = chunk[blockDim.x];
+    if (threadIdx.x == 0) send_offset[experts] = chunk[32];
     if (peer_offset && !peer_to_pool) {
         // Where this rank's rows for global expert ge start in the RECEIVE buffer of the rank that owns ge
         // (source-major there): rows of lower-ranked sources for that destination, then this rank's rows
@@ -143,14 +157,16 @@ __global__ void plan_kernel(int* __restrict__ block_valid, int* counts, int worl
     __syncthreads();
     // 2. segments (source rank r, local expert e) in the receive buffer: source-major, expert order inside
     //    a source, which is the order pack() wrote them
-    for (int i = threadIdx.x; i < segments; i += blockDim.x) {
-        const int r = i / local_experts, e = i - r * local_experts;
-        scan[i] = counts[r * experts + rank * local_experts + e];
+    if (world > 1) {                                      // (one rank: what the first scan left)
+        for (int i = threadIdx.x; i < segments; i += blockDim.x) {
+            const int r = i / local_experts, e = i - r * local_experts;
+            scan[i] = counts[r * experts + rank * local_experts + e];
+        }
+        __syncthreads();
+        block_exclusive_scan(scan, segments, chunk);
     }
-    __syncthreads();
-    block_exclusive_scan(scan, segments, chunk);
     for (int i = threadIdx.x; i < segments; i += blockDim.x) seg_src_offset[i] = scan[i];
-    if (threadIdx.x == 0) { seg_src_offset[segments] = chunk[blockDim.x]; totals[0] = chunk[blockDim.x]; }
+    if (threadIdx.x == 0) { seg_src_offset[segments] = chunk[32]; totals[0] = chunk[32]; }
     __syncthreads();
     // 3. expert-major pool, every expert padded to whole blocks of block_rows (128 or 256) rows
     for (int e = threadIdx.x; e < local_experts; e += blockDim.x) {
@@ -160,7 +176,7 @@ __global__ void plan_kernel(int* __restrict__ block_valid, int* counts, int worl
     }
     __syncthreads();
     block_exclusive_scan(scan, local_experts, chunk);
-    const int pool_rows = chunk[blockDim.x];
+    const int pool_rows = chunk[32];
     const bool overflow = pool_rows > capacity_rows;
     for (int e = threadIdx.x; e < local_experts; e += blockDim.x) {
         pool_off[e] = scan[e];
@@ -668,7 +684,7 @@ void moe_plan(int* block_valid, int* counts_matrix, int world, int rank, int exp
     if (block_rows != 128 && block_rows != 256) throw std::invalid_argument("moe plan: block rows must be 128 or 256");
     if (pool_capacity_rows <= 0 || pool_capacity_rows % block_rows) throw std::invalid_argument("moe plan: pool capacity must be a multiple of the block rows");
     const int local = experts / world;
-    launch_chained(plan_kernel, dim3(1), dim3(256), size_t((experts + local + 257) * sizeof(int)), stream, block_valid, counts_matrix, world, rank, experts, pool_capacity_rows, block_rows,
+    launch_chained(plan_kernel, dim3(1), dim3(PLAN_THREADS), size_t((experts + local + 33) * sizeof(int)), stream, block_valid, counts_matrix, world, rank, experts, pool_capacity_rows, block_rows,
                                                                    send_offset, seg_src_offset, seg_pool_offset,
                                                                    block_expert, num_blocks, totals, peer_offset, ids, routes, cursor, peer_to_pool);
 }

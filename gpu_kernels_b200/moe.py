@@ -222,9 +222,9 @@ class Nvfp4MoE:
     def _metadata(self, ids, tokens, block_rows):
         lib, s = _lib.load(), _stream()
         routes = tokens * self.topk
-        if self.world == 1 and routes <= 4096:
-            # one launch: histogram of the routes (by the plan's single CTA: for small batches), plan, arrival
-            # counters cleared
+        if self.world == 1 and routes <= 32768:
+            # one launch: histogram of the routes (by the plan's single CTA: 24576 routes take it less time than
+            # clearing, counting and copying as launches of their own), plan, arrival counters cleared
             _lib.check(lib.gpu_kernels_nvfp4_moe_route_plan(
                 ids.data_ptr(), routes, self.counts_matrix.data_ptr(), self.experts, self.pool_rows, block_rows,
                 self.send_offset.data_ptr(), self.seg_src.data_ptr(), self.seg_pool.data_ptr(),
@@ -252,10 +252,13 @@ class Nvfp4MoE:
                 self.block_expert.data_ptr(), self.num_blocks.data_ptr(), self.totals.data_ptr(),
                 self.peer_offset.data_ptr() if self._peer is not None else None, 1 if self.to_pool else 0,
                 self.cursor.data_ptr(), self.block_valid.data_ptr(), s))
-        # padding rows of the live blocks must contribute nothing: clear their scale bytes, weights and codes
-        _lib.check(lib.gpu_kernels_nvfp4_moe_clear_live(
-            self.num_blocks.data_ptr(), block_rows, self.pool_rows, self.hidden, self.pool_scales.data_ptr(),
-            self.pool_weight.data_ptr(), self.pool_dst.data_ptr() if self._peer is not None else None, s))
+        # Padding rows of the live blocks must contribute nothing: clear their scale bytes, weights and codes. On one
+        # rank with the fused epilogues nothing reads them: a row of a product depends on its own row of A alone, and
+        # both GEMMs store only the rows block_valid counts, so the launch (3.5 us) is left out.
+        if self.world > 1 or not self.fused:
+            _lib.check(lib.gpu_kernels_nvfp4_moe_clear_live(
+                self.num_blocks.data_ptr(), block_rows, self.pool_rows, self.hidden, self.pool_scales.data_ptr(),
+                self.pool_weight.data_ptr(), self.pool_dst.data_ptr() if self._peer is not None else None, s))
         if self._peer is not None and self.pool_rows >= self.world * self.max_tokens * self.topk + self.local_experts * (block_rows - 1):
             # peer exchange with a worst-case pool: the host needs nothing from the counts
             return None, None

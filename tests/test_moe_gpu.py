@@ -397,3 +397,35 @@ def test_nothing_the_layer_reads_is_left_over_from_before(g, fused, block_rows):
         layer.check()
         assert_layer_close(y, oracle_layer(x[:tokens], ids, wts, w1, w2, 10.0), f"poisoned buffers, T={tokens}")
     layer.close()
+
+
+@pytest.mark.parametrize("experts,routes,block_rows", [(1, 6, 128), (33, 5000, 128), (256, 24576, 256), (1000, 32768, 128), (4096, 4097, 128)])
+def test_route_plan_of_one_rank(g, experts, routes, block_rows):
+    # histogram, the scans (fewer experts than threads, more, odd counts) and the block tables, exact
+    from gpu_kernels_b200 import _lib
+    rng = np.random.default_rng(experts + routes)
+    ids = rng.integers(-1, experts, routes)                                 # -1: dropped routes
+    if experts > 1:
+        ids[rng.random(routes) < 0.3] = experts // 2                        # one popular expert
+    counts = np.bincount(ids[ids >= 0], minlength=experts)
+    padded = (counts + block_rows - 1) // block_rows * block_rows
+    rows = int(padded.sum())
+    capacity = rows + 2 * block_rows
+    i32 = lambda n: torch.full((n,), -7, dtype=torch.int32, device="cuda")
+    c, send, src, pool, be, nb, tot, cur, bv = (i32(n) for n in (experts, experts + 1, experts + 1, experts, capacity // block_rows, 1, 4,
+                                                                 experts, capacity // block_rows))
+    t = torch.from_numpy(ids).cuda()
+    _lib.check(_lib.load().gpu_kernels_nvfp4_moe_route_plan(
+        t.data_ptr(), routes, c.data_ptr(), experts, capacity, block_rows, send.data_ptr(), src.data_ptr(), pool.data_ptr(), be.data_ptr(),
+        nb.data_ptr(), tot.data_ptr(), cur.data_ptr(), bv.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    start = np.concatenate(([0], np.cumsum(counts)))
+    first = np.cumsum(padded) - padded
+    blocks = rows // block_rows
+    assert np.array_equal(to_np(c), counts) and not to_np(cur).any()
+    assert np.array_equal(to_np(send), start) and np.array_equal(to_np(src), start)
+    assert np.array_equal(to_np(pool), first)
+    assert to_np(nb)[0] == blocks and to_np(tot)[:3].tolist() == [counts.sum(), rows, 0]
+    owner = np.repeat(np.arange(experts), padded // block_rows)
+    assert np.array_equal(to_np(be)[:blocks], owner) and (to_np(be)[blocks:] == -7).all()
+    left = (first + counts)[owner] - np.arange(blocks) * block_rows
+    assert np.array_equal(to_np(bv)[:blocks], np.clip(left, 0, block_rows))
