@@ -1428,7 +1428,8 @@ void launch_dense(const gpu_kernels::Nvfp4Params& p, const CUtensorMap& tmC, con
         // MXFP4 plans have the masked register-store route only
         if (p.split_k > 1 || p.gather_world || g.prof) throw std::invalid_argument("mxfp4 gemm: plain launches only");
         launch_instance<CG, UN, EPI_DIRECT_EDGE, false, true>(dev, units, p.A, p.B, p.SFA, p.SFB, tmC, g, stream, pdl);
-    } else if (p.M % 128 || p.N % 128) {
+    } else if (p.M % 128 || p.N % 128 || (!g.c_rows_32 && p.split_k <= 1 && !p.gather_world && !staged && !g.prof)) {
+        // masked, and in 16-byte stores where C itself does not start on a 32-byte boundary
         if (p.split_k > 1 || p.gather_world || g.prof) throw std::invalid_argument("nvfp4 gemm: M or N is no multiple of 128: plain launches only");
         launch_instance<CG, UN, EPI_DIRECT_EDGE>(dev, units, p.A, p.B, p.SFA, p.SFB, tmC, g, stream, pdl);
     } else if (p.split_k > 1) {
@@ -1475,6 +1476,8 @@ void launch_plain(const gpu_kernels::Nvfp4Params& p, const CUtensorMap& tmC, con
 void launch_with(const gpu_kernels::Nvfp4Params& p, void* C, cudaStream_t stream, unsigned long long* prof) {
     if (!C || (reinterpret_cast<uintptr_t>(C) & 15)) throw std::invalid_argument("nvfp4 gemm: C must be 16-byte aligned");
     if (prof && (p.split_k > 1 || p.gather_world)) throw std::invalid_argument("nvfp4 gemm profile: plain plans only");
+    if ((reinterpret_cast<uintptr_t>(C) & 31) && (p.split_k > 1 || (prof && p.direct_store)))
+        throw std::invalid_argument("nvfp4 gemm: split-K and profiled launches store 32 bytes at a time: C must be 32-byte aligned");
     const CUtensorMap tmC = output_map(C, p.M, p.N, p.out_bf16 != 0);
     const GemmArgs g = dense_args(p, C, prof);
     if (p.plain_tile_n && p.split_k <= 1 && !p.gather_world && !p.ragged_units && !p.route && p.direct_store && !prof) {

@@ -468,6 +468,22 @@ def test_plain_launch_on_other_tiles(g, m, n, k, variant):
     plan.close()
 
 
+@pytest.mark.parametrize("m,n,k", [(128, 256, 2048), (256, 512, 256), (384, 640, 512)])
+def test_output_that_starts_on_a_16_byte_boundary(g, m, n, k):
+    # whole tiles into a C that is 16- but not 32-byte aligned: the same bits as into an aligned one
+    pa, sa = g.quantize(random_operand(m, k, seed=m))
+    pb, sb = g.quantize(random_operand(n, k, seed=n, scale=0.05))
+    plan = g.Nvfp4Gemm(pa, pb, sa, sb)
+    aligned = plan.run()
+    flat = torch.full((m * n + 16,), 77.0, dtype=torch.float16, device="cuda")
+    out = flat[8:8 + m * n].view(m, n)
+    assert out.data_ptr() % 32 == 16
+    plan.run(out)
+    plan.validate()
+    assert torch.equal(out, aligned) and bool((flat[:8] == 77.0).all()) and bool((flat[8 + m * n:] == 77.0).all())
+    plan.close()
+
+
 def test_mxfp4_edge_shapes(g):
     for m, n, k in [(1, 264, 256), (100, 200, 512), (500, 1000, 384)]:
         a = random_operand(m, k, seed=m + k)
