@@ -4,6 +4,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <cstdlib>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -14,6 +15,25 @@ enum InputDtype : int { DTYPE_BF16 = 0, DTYPE_F16 = 1, DTYPE_F32 = 2 };
 
 inline void cuda_check(cudaError_t e) {
     if (e != cudaSuccess) throw std::runtime_error(std::string("CUDA: ") + cudaGetErrorString(e));
+}
+
+// Launch with the programmatic stream-serialisation attribute: the kernel may be scheduled while the one in front of it
+// in the stream drains, and waits (griddepcontrol.wait) before it touches global memory. NVFP4_B200_PDL=0 launches the
+// ordinary way.
+template <typename... Params, typename... Args>
+void launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+    static const bool pdl = [] { const char* v = std::getenv("NVFP4_B200_PDL"); return !(v && v[0] == '0'); }();
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    cuda_check(cudaLaunchKernelEx(&cfg, kernel, Params(args)...));
 }
 
 // Refuse to run on anything but a compute-capability 10.x device: there is no

@@ -44,22 +44,6 @@ __device__ __forceinline__ void chain_point() {
     ptx::grid_dependency_wait();
 }
 
-template <typename... Params, typename... Args>
-void launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
-    static const bool pdl = [] { const char* v = std::getenv("NVFP4_B200_PDL"); return !(v && v[0] == '0'); }();
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cfg.attrs = &attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    cuda_check(cudaLaunchKernelEx(&cfg, kernel, Params(args)...));
-}
-
 __global__ void route_count_kernel(const long long* __restrict__ ids, int routes, int experts, int* __restrict__ counts) {
     chain_point();
     extern __shared__ int local[];
