@@ -32,32 +32,36 @@ __device__ __forceinline__ void chain_point() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-template <typename T> struct Loader;
-template <> struct Loader<float> {
-    static __device__ __forceinline__ void load(const float* p, float (&v)[16]) {
-        #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float4 f = __ldg(reinterpret_cast<const float4*>(p) + i);
-            v[4 * i] = f.x; v[4 * i + 1] = f.y; v[4 * i + 2] = f.z; v[4 * i + 3] = f.w;
-        }
-    }
-};
-
 template <typename T> struct PairFormat { using type = void; };
 template <> struct PairFormat<__nv_bfloat16> { using type = Bf16Pairs; };
 template <> struct PairFormat<__half> { using type = Fp16Pairs; };
 
-// One block of 16 values straight from global memory to its scale byte and packed codes.
-template <typename T>
-__device__ __forceinline__ uint32_t quantise_from(const T* p, uint2& out) {
-    if constexpr (sizeof(T) == 2) {
-        const uint4 a = __ldg(reinterpret_cast<const uint4*>(p));
-        const uint4 b = __ldg(reinterpret_cast<const uint4*>(p) + 1);
-        const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+// One block of 16 values, as loaded, to its scale byte and packed codes. SCALED: every value times inv_global, in
+// FP32, first (the product is no longer a 16-bit value, so it takes the FP32 routine whatever the input type).
+template <typename T, bool SCALED>
+__device__ __forceinline__ uint32_t quantise_raw(const uint4 (&raw)[sizeof(T)], float inv_global, uint2& out) {
+    if constexpr (sizeof(T) == 2 && !SCALED) {
+        const uint32_t w[8] = {raw[0].x, raw[0].y, raw[0].z, raw[0].w, raw[1].x, raw[1].y, raw[1].z, raw[1].w};
         return quantise_block_pairs<typename PairFormat<T>::type>(w, out);
     } else {
         float v[16];
-        Loader<T>::load(p, v);
+        #pragma unroll
+        for (int i = 0; i < int(sizeof(T)); ++i) {
+            const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+            #pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if constexpr (sizeof(T) == 4) {
+                    v[4 * i + j] = __uint_as_float(w[j]);
+                } else {
+                    v[8 * i + 2 * j] = PairFormat<T>::type::widen(w[j] & 0xFFFFu);
+                    v[8 * i + 2 * j + 1] = PairFormat<T>::type::widen(w[j] >> 16);
+                }
+            }
+        }
+        if constexpr (SCALED) {
+            #pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = __fmul_rn(v[i], inv_global);
+        }
         return quantise_block<true>(v, out);
     }
 }
@@ -70,10 +74,12 @@ __device__ __forceinline__ uint32_t quantise_from(const T* p, uint2& out) {
 // TAIL: the instance for a tensor whose last row tile is partial (rows % 128 != 0): rows the tensor does not have are
 // read as zeros, which gives them the scale byte of a zero block (0x01) in the atom and no packed bytes. One launch for
 // all row tiles: the last one as a launch of its own cost 1000 x 8192 bf16 another 4 us behind the 7 us of the others.
-template <typename T, int COLS, bool TAIL = false>
+// SCALED (two-level scaling): the values are first multiplied by the reciprocal of a per-tensor scale; the GEMM undoes
+// the tensor scales through its alpha.
+template <typename T, int COLS, bool TAIL, bool SCALED>
 __global__ void __launch_bounds__(Q_THREADS, 4)
 quantise_kernel(const T* __restrict__ x, uint8_t* __restrict__ packed, uint8_t* __restrict__ scales,
-                int rows, int K) {
+                int rows, int K, float inv_global) {
     chain_point();
     constexpr int BLOCKS = COLS / 16;                           // 16-value blocks across the tile
     constexpr int ROWS_PER_PASS = Q_THREADS / BLOCKS;
@@ -93,42 +99,29 @@ quantise_kernel(const T* __restrict__ x, uint8_t* __restrict__ packed, uint8_t* 
             *reinterpret_cast<uint2*>(packed + size_t(row_base + r) * (K / 2) + k / 2) = out;
         sf_tile[(kb >> 2) * 512 + (r & 31) * 16 + (r >> 5) * 4 + (kb & 3)] = static_cast<uint8_t>(sbyte);
     };
-    if constexpr (sizeof(T) == 2) {
-        // 16-bit inputs: the loads of two passes are kept in flight ahead of the arithmetic (32 bytes per thread
-        // and pass), so that a warp waits for memory once per tile rather than once per pass.
-        constexpr int AHEAD = 2;
-        uint4 lo[AHEAD], hi[AHEAD];
-        auto fetch = [&](int pass, uint4& a, uint4& b) {
-            const int r = pass * ROWS_PER_PASS + row_in_pass;
-            const uint4* p = reinterpret_cast<const uint4*>(x + size_t(row_base + r) * K + k);
-            if (TAIL && row_base + r >= rows) { a = b = make_uint4(0u, 0u, 0u, 0u); return; }
-            a = __ldg(p);
-            b = __ldg(p + 1);
-        };
-        if (live) {
-            #pragma unroll
-            for (int i = 0; i < AHEAD; ++i) fetch(i, lo[i], hi[i]);
-            #pragma unroll
-            for (int pass = 0; pass < PASSES; ++pass) {
-                const uint4 a = lo[pass % AHEAD], b = hi[pass % AHEAD];
-                if (pass + AHEAD < PASSES) fetch(pass + AHEAD, lo[pass % AHEAD], hi[pass % AHEAD]);
-                const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-                uint2 out;
-                const uint32_t sbyte = quantise_block_pairs<typename PairFormat<T>::type>(w, out);
-                emit(pass * ROWS_PER_PASS + row_in_pass, sbyte, out);
-            }
-        }
-    } else {
-        #pragma unroll 4
+    // The loads of the next passes are kept in flight ahead of the arithmetic, so that a warp waits for memory once per
+    // tile rather than once per pass: two passes for 16-bit inputs (32 bytes per thread and pass), one for FP32 (64).
+    constexpr int WORDS = int(sizeof(T)), AHEAD = sizeof(T) == 2 ? 2 : 1;
+    uint4 raw[AHEAD][WORDS];
+    auto fetch = [&](int pass, uint4 (&to)[WORDS]) {
+        const int r = pass * ROWS_PER_PASS + row_in_pass;
+        const uint4* p = reinterpret_cast<const uint4*>(x + size_t(row_base + r) * K + k);
+        const bool there = !TAIL || row_base + r < rows;
+        #pragma unroll
+        for (int i = 0; i < WORDS; ++i) to[i] = there ? __ldg(p + i) : make_uint4(0u, 0u, 0u, 0u);
+    };
+    if (live) {
+        #pragma unroll
+        for (int i = 0; i < AHEAD; ++i) fetch(i, raw[i]);
+        #pragma unroll
         for (int pass = 0; pass < PASSES; ++pass) {
-            const int r = pass * ROWS_PER_PASS + row_in_pass;
-            if (live) {
-                uint2 out;
-                uint32_t sbyte = 0x01u;
-                if (TAIL && row_base + r >= rows) out = make_uint2(0u, 0u);
-                else sbyte = quantise_from(x + size_t(row_base + r) * K + k, out);
-                emit(r, sbyte, out);
-            }
+            uint4 now[WORDS];
+            #pragma unroll
+            for (int i = 0; i < WORDS; ++i) now[i] = raw[pass % AHEAD][i];
+            if (pass + AHEAD < PASSES) fetch(pass + AHEAD, raw[pass % AHEAD]);
+            uint2 out;
+            const uint32_t sbyte = quantise_raw<T, SCALED>(now, inv_global, out);
+            emit(pass * ROWS_PER_PASS + row_in_pass, sbyte, out);
         }
     }
     __syncthreads();
@@ -138,55 +131,6 @@ quantise_kernel(const T* __restrict__ x, uint8_t* __restrict__ packed, uint8_t* 
         const size_t first_atom = size_t(row_tile) * (K / 64) + size_t(blockIdx.x) * ATOMS;
         reinterpret_cast<uint4*>(scales + first_atom * 512)[threadIdx.x] =
             reinterpret_cast<const uint4*>(sf_tile)[threadIdx.x];
-    }
-}
-
-// Two-level scaling: every value is first multiplied (in FP32) by the reciprocal of a per-tensor scale, then
-// quantised as above; the GEMM undoes the tensor scales through its alpha. One 16-value block per thread and pass,
-// through the FP32 block routine whatever the input type (the product is no longer a 16-bit value).
-template <typename T>
-__global__ void __launch_bounds__(Q_THREADS)
-quantise_scaled_kernel(const T* __restrict__ x, float inv_global, uint8_t* __restrict__ packed,
-                       uint8_t* __restrict__ scales, int rows, int K) {
-    chain_point();
-    __shared__ __align__(16) uint8_t sf_tile[4 * 512];
-    const int kb = threadIdx.x & 15, row_in_pass = threadIdx.x >> 4;
-    const int col0 = blockIdx.x * 256, row_base = blockIdx.y * Q_ROWS;
-    const int k = col0 + kb * 16;
-    if (k < K) {
-        #pragma unroll 2
-        for (int pass = 0; pass < 8; ++pass) {
-            const int r = pass * 16 + row_in_pass;
-            const T* p = x + size_t(row_base + r) * K + k;
-            if (row_base + r >= rows) {                         // a row the tensor does not have: a zero block's scale
-                sf_tile[(kb >> 2) * 512 + (r & 31) * 16 + (r >> 5) * 4 + (kb & 3)] = 0x01u;
-                continue;
-            }
-            float v[16];
-            if constexpr (sizeof(T) == 4) {
-                Loader<float>::load(reinterpret_cast<const float*>(p), v);
-            } else {
-                const uint4 a = __ldg(reinterpret_cast<const uint4*>(p)), b = __ldg(reinterpret_cast<const uint4*>(p) + 1);
-                const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-                #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    v[2 * i] = PairFormat<T>::type::widen(w[i] & 0xFFFFu);
-                    v[2 * i + 1] = PairFormat<T>::type::widen(w[i] >> 16);
-                }
-            }
-            #pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = __fmul_rn(v[i], inv_global);
-            uint2 out;
-            const uint32_t sbyte = quantise_block<true>(v, out);
-            *reinterpret_cast<uint2*>(packed + size_t(row_base + r) * (K / 2) + k / 2) = out;
-            sf_tile[(kb >> 2) * 512 + (r & 31) * 16 + (r >> 5) * 4 + (kb & 3)] = static_cast<uint8_t>(sbyte);
-        }
-    }
-    __syncthreads();
-    const int atoms = min(4, (K - col0) / 64);
-    if (int(threadIdx.x) < atoms * 32) {
-        const size_t first_atom = size_t(blockIdx.y) * (K / 64) + size_t(blockIdx.x) * 4;
-        reinterpret_cast<uint4*>(scales + first_atom * 512)[threadIdx.x] = reinterpret_cast<const uint4*>(sf_tile)[threadIdx.x];
     }
 }
 
@@ -321,11 +265,11 @@ void check_quant_shape(int rows, int K) {
     if (K % 64 != 0) throw std::invalid_argument("nvfp4 quantise: K must be a multiple of 64");
 }
 
-void quantise(const void* x, int dtype, uint8_t* packed, uint8_t* scales, int rows, int K, cudaStream_t stream) {
-    check_quant_shape(rows, K);
-    if (!x || !packed || !scales) throw std::invalid_argument("nvfp4 quantise: null pointer");
-    if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(packed) | reinterpret_cast<uintptr_t>(scales)) & 15)
-        throw std::invalid_argument("nvfp4 quantise: pointers must be 16-byte aligned");
+namespace {
+
+template <bool SCALED>
+void launch_quantise(const void* x, int dtype, float inv_global, uint8_t* packed, uint8_t* scales, int rows, int K,
+                     cudaStream_t stream) {
     // 256-column tiles; 128-column ones when the grid would otherwise be less than two waves of resident CTAs
     // (four per SM). Measured, 128 / 256 columns: 4096 x 4096 bf16 12.3 / 14.4 us, 8192 x 8192 36.9 / 34.0 us.
     int device = 0, sms = 0;
@@ -335,14 +279,15 @@ void quantise(const void* x, int dtype, uint8_t* packed, uint8_t* scales, int ro
     const bool narrow = K % 128 == 0 && wide_ctas < 2LL * 4 * sms;
     auto launch = [&](auto tag) {
         using T = decltype(tag);
-        const auto* in = static_cast<const T*>(x);
         const int cols = narrow ? 128 : 256;
         const int row_tiles = (rows + Q_ROWS - 1) / Q_ROWS;
         const dim3 grid((K + cols - 1) / cols, std::min(row_tiles, MAX_GRID_Y), (row_tiles + MAX_GRID_Y - 1) / MAX_GRID_Y);
-        auto go = [&](auto kernel) { launch_chained(kernel, grid, dim3(Q_THREADS), size_t(0), stream, in, packed, scales, rows, K); };
+        auto go = [&](auto kernel) {
+            launch_chained(kernel, grid, dim3(Q_THREADS), size_t(0), stream, static_cast<const T*>(x), packed, scales, rows, K, inv_global);
+        };
         const bool tail = rows % Q_ROWS != 0;
-        if (narrow) tail ? go(quantise_kernel<T, 128, true>) : go(quantise_kernel<T, 128>);
-        else tail ? go(quantise_kernel<T, 256, true>) : go(quantise_kernel<T, 256>);
+        if (narrow) tail ? go(quantise_kernel<T, 128, true, SCALED>) : go(quantise_kernel<T, 128, false, SCALED>);
+        else tail ? go(quantise_kernel<T, 256, true, SCALED>) : go(quantise_kernel<T, 256, false, SCALED>);
     };
     switch (dtype) {
         case DTYPE_BF16: launch(__nv_bfloat16{}); break;
@@ -354,28 +299,26 @@ void quantise(const void* x, int dtype, uint8_t* packed, uint8_t* scales, int ro
     cuda_check(cudaGetLastError());
 }
 
-void quantise_scaled(const void* x, int dtype, float inv_global, uint8_t* packed, uint8_t* scales, int rows, int K,
-                     cudaStream_t stream) {
-    check_quant_shape(rows, K);
+void check_quant_pointers(const void* x, const uint8_t* packed, const uint8_t* scales) {
     if (!x || !packed || !scales) throw std::invalid_argument("nvfp4 quantise: null pointer");
     if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(packed) | reinterpret_cast<uintptr_t>(scales)) & 15)
         throw std::invalid_argument("nvfp4 quantise: pointers must be 16-byte aligned");
+}
+
+}  // namespace
+
+void quantise(const void* x, int dtype, uint8_t* packed, uint8_t* scales, int rows, int K, cudaStream_t stream) {
+    check_quant_shape(rows, K);
+    check_quant_pointers(x, packed, scales);
+    launch_quantise<false>(x, dtype, 1.0f, packed, scales, rows, K, stream);
+}
+
+void quantise_scaled(const void* x, int dtype, float inv_global, uint8_t* packed, uint8_t* scales, int rows, int K,
+                     cudaStream_t stream) {
+    check_quant_shape(rows, K);
+    check_quant_pointers(x, packed, scales);
     if (!(inv_global > 0.0f) || !(inv_global < 3.0e38f)) throw std::invalid_argument("nvfp4 quantise: the tensor scale must be positive and finite");
-    const dim3 grid((K + 255) / 256, (rows + Q_ROWS - 1) / Q_ROWS);
-    switch (dtype) {
-        case DTYPE_BF16:
-            launch_chained(quantise_scaled_kernel<__nv_bfloat16>, grid, dim3(Q_THREADS), size_t(0), stream, static_cast<const __nv_bfloat16*>(x), inv_global, packed, scales, rows, K);
-            break;
-        case DTYPE_F16:
-            launch_chained(quantise_scaled_kernel<__half>, grid, dim3(Q_THREADS), size_t(0), stream, static_cast<const __half*>(x), inv_global, packed, scales, rows, K);
-            break;
-        case DTYPE_F32:
-            launch_chained(quantise_scaled_kernel<float>, grid, dim3(Q_THREADS), size_t(0), stream, static_cast<const float*>(x), inv_global, packed, scales, rows, K);
-            break;
-        default:
-            throw std::invalid_argument("nvfp4 quantise: dtype must be 0 (bf16), 1 (fp16) or 2 (fp32)");
-    }
-    cuda_check(cudaGetLastError());
+    launch_quantise<true>(x, dtype, inv_global, packed, scales, rows, K, stream);
 }
 
 void check_mx_shape(int rows, int K) {
