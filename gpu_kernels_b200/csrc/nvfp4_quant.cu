@@ -171,68 +171,73 @@ dequantise_kernel(const uint8_t* __restrict__ packed, const uint8_t* __restrict_
 // Per block: e = floor(log2(amax)) - 2 (2 = the largest exponent of E2M1), clamped to [-127, 127]; scale byte
 // e + 127; q = x * 2^-e (exact but for underflow) encoded as E2M1 with the quantiser's rounding and sign rule.
 // An all-zero block takes e = -127; a block with a NaN or an infinity takes the NaN scale 0xFF and the codes of
-// the NVFP4 NaN block. One thread per block. The scale bytes go to cuBLASLt's VEC32 order: the VEC16 atoms with
-// K/32 blocks per row.
+// the NVFP4 NaN block. The scale bytes go to cuBLASLt's VEC32 order: the VEC16 atoms with K/32 blocks per row.
+// A CTA owns one scale atom, 128 rows x 128 columns: two blocks of 32 per thread, the second's loads in flight during the
+// first's arithmetic (16-bit inputs), the atom's bytes gathered in shared memory and written as one run (one thread per
+// block, each scale byte stored by itself: see the commit that replaced it for the figures).
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(Q_THREADS, sizeof(T) == 2 ? 4 : 3)
 quantise_mx_kernel(const T* __restrict__ x, uint8_t* __restrict__ packed, uint8_t* __restrict__ scales, int rows, int K) {
-    const size_t idx = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    const int blocks_per_row = K / 32;
-    if (idx >= size_t((rows + 127) / 128 * 128) * blocks_per_row) return;
-    const int r = int(idx / blocks_per_row), b = int(idx % blocks_per_row);
-    if (r >= rows) {                                            // a row the tensor does not have: a zero block's scale
-        scales[scale_byte_offset(r, b, K / 2)] = 0u;
-        return;
+    chain_point();
+    constexpr int WORDS = 2 * int(sizeof(T));                  // 16-byte words of a block
+    __shared__ __align__(16) uint8_t sf_tile[512];
+    const int kb = threadIdx.x & 3, row_in_pass = threadIdx.x >> 2, row_base = int(blockIdx.x / unsigned(K / 128)) * Q_ROWS;
+    const size_t k = size_t(blockIdx.x % unsigned(K / 128)) * 128 + kb * 32;
+    uint4 raw[2][WORDS];
+    #pragma unroll
+    for (int pass = 0; pass < 2; ++pass) {
+        const int row = row_base + pass * 64 + row_in_pass;
+        const uint4* p = reinterpret_cast<const uint4*>(x + size_t(row) * K + k);
+        #pragma unroll
+        for (int i = 0; i < WORDS; ++i) raw[pass][i] = row < rows ? __ldg(p + i) : make_uint4(0u, 0u, 0u, 0u);
     }
-    const T* p = x + size_t(r) * K + size_t(b) * 32;
-    float v[32];
-    if constexpr (sizeof(T) == 4) {
+    #pragma unroll
+    for (int pass = 0; pass < 2; ++pass) {
+        const int r = pass * 64 + row_in_pass;
+        float v[32];
         #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float4 f = __ldg(reinterpret_cast<const float4*>(p) + i);
-            v[4 * i] = f.x; v[4 * i + 1] = f.y; v[4 * i + 2] = f.z; v[4 * i + 3] = f.w;
-        }
-    } else {
-        #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint4 a = __ldg(reinterpret_cast<const uint4*>(p) + i);
-            const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+        for (int i = 0; i < WORDS; ++i) {
+            const uint32_t w[4] = {raw[pass][i].x, raw[pass][i].y, raw[pass][i].z, raw[pass][i].w};
             #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                v[8 * i + 2 * j] = PairFormat<T>::type::widen(w[j] & 0xFFFFu);
-                v[8 * i + 2 * j + 1] = PairFormat<T>::type::widen(w[j] >> 16);
+                if constexpr (sizeof(T) == 4) {
+                    v[4 * i + j] = __uint_as_float(w[j]);
+                } else {
+                    v[8 * i + 2 * j] = PairFormat<T>::type::widen(w[j] & 0xFFFFu);
+                    v[8 * i + 2 * j + 1] = PairFormat<T>::type::widen(w[j] >> 16);
+                }
             }
         }
-    }
-    uint32_t mx = 0;
-    #pragma unroll
-    for (int i = 0; i < 32; ++i) mx = max(mx, __float_as_uint(v[i]) & 0x7FFFFFFFu);
-    uint4* out = reinterpret_cast<uint4*>(packed + size_t(r) * (K / 2) + size_t(b) * 16);
-    // the scale of (row, block of 32) sits where the VEC16 layout of a K/2-wide tensor puts (row, block of 16)
-    uint8_t* sbyte = scales + scale_byte_offset(r, b, K / 2);
-    if (mx >= 0x7F800000u) {
-        *out = make_uint4(0x77777777u, 0x77777777u, 0x77777777u, 0x77777777u);
-        *sbyte = 0xFFu;
-        return;
-    }
-    int e = mx ? ilogbf(__uint_as_float(mx)) - 2 : -127;
-    e = min(max(e, -127), 127);
-    const float inv = scalbnf(1.0f, -e);
-    uint32_t words[4];
-    #pragma unroll
-    for (int h = 0; h < 4; ++h) {
-        float q[8];
-        uint32_t signs = 0;
+        uint32_t mx = 0;
         #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float t = __fmul_rn(v[8 * h + i], inv);
-            q[i] = fabsf(t);
-            signs |= t < 0.0f ? (8u << (4 * i)) : 0u;
+        for (int i = 0; i < 32; ++i) mx = max(mx, __float_as_uint(v[i]) & 0x7FFFFFFFu);
+        uint32_t words[4] = {0x77777777u, 0x77777777u, 0x77777777u, 0x77777777u}, sbyte = 0xFFu;
+        if (mx < 0x7F800000u) {
+            // floor(log2(amax)) is the exponent field; zero and subnormal maxima end at the clamp either way
+            const int e = max(int(mx >> 23) - 129, -127);
+            const float inv = __uint_as_float(uint32_t(127 - e) << 23);
+            #pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                float q[8];
+                uint32_t signs = 0;
+                #pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float t = __fmul_rn(v[8 * h + i], inv);
+                    q[i] = fabsf(t);
+                    signs |= t < 0.0f ? (8u << (4 * i)) : 0u;
+                }
+                words[h] = e2m1x8_from_quotients(q) | signs;
+            }
+            sbyte = uint32_t(e + 127);
         }
-        words[h] = e2m1x8_from_quotients(q) | signs;
+        if (row_base + r < rows)
+            *reinterpret_cast<uint4*>(packed + size_t(row_base + r) * (K / 2) + k / 2) = make_uint4(words[0], words[1], words[2], words[3]);
+        sf_tile[(r & 31) * 16 + (r >> 5) * 4 + kb] = static_cast<uint8_t>(sbyte);     // a row the tensor does not have: a zero block's 0
     }
-    *out = make_uint4(words[0], words[1], words[2], words[3]);
-    *sbyte = static_cast<uint8_t>(e + 127);
+    __syncthreads();
+    if (threadIdx.x < 32)
+        reinterpret_cast<uint4*>(scales + size_t(blockIdx.x) * 512)[threadIdx.x] =
+            reinterpret_cast<const uint4*>(sf_tile)[threadIdx.x];
 }
 
 // MXFP4 bytes -> FP32 [rows, K]; one thread per block of 32 (the check path).
@@ -331,12 +336,15 @@ void quantise_mx(const void* x, int dtype, uint8_t* packed, uint8_t* scales, int
     if (!x || !packed || !scales) throw std::invalid_argument("mxfp4 quantise: null pointer");
     if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(packed) | reinterpret_cast<uintptr_t>(scales)) & 15)
         throw std::invalid_argument("mxfp4 quantise: pointers must be 16-byte aligned");
-    const size_t blocks = size_t((rows + 127) / 128 * 128) * (K / 32);    // the rows of the last atom the tensor lacks get their scale byte
-    const unsigned grid = static_cast<unsigned>((blocks + 255) / 256);
+    const dim3 grid(unsigned(K / 128) * unsigned((rows + Q_ROWS - 1) / Q_ROWS));
+    auto launch = [&](auto tag) {
+        using T = decltype(tag);
+        launch_chained(quantise_mx_kernel<T>, grid, dim3(Q_THREADS), size_t(0), stream, static_cast<const T*>(x), packed, scales, rows, K);
+    };
     switch (dtype) {
-        case DTYPE_BF16: quantise_mx_kernel<<<grid, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), packed, scales, rows, K); break;
-        case DTYPE_F16: quantise_mx_kernel<<<grid, 256, 0, stream>>>(static_cast<const __half*>(x), packed, scales, rows, K); break;
-        case DTYPE_F32: quantise_mx_kernel<<<grid, 256, 0, stream>>>(static_cast<const float*>(x), packed, scales, rows, K); break;
+        case DTYPE_BF16: launch(__nv_bfloat16{}); break;
+        case DTYPE_F16: launch(__half{}); break;
+        case DTYPE_F32: launch(float{}); break;
         default: throw std::invalid_argument("mxfp4 quantise: dtype must be 0 (bf16), 1 (fp16) or 2 (fp32)");
     }
     cuda_check(cudaGetLastError());
