@@ -62,7 +62,7 @@ __device__ __forceinline__ uint32_t quantise_raw(const uint4 (&raw)[sizeof(T)], 
             #pragma unroll
             for (int i = 0; i < 16; ++i) v[i] = __fmul_rn(v[i], inv_global);
         }
-        return quantise_block<true>(v, out);
+        return quantise_block(v, out);
     }
 }
 

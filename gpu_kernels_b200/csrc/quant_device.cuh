@@ -58,10 +58,9 @@ __device__ __forceinline__ uint32_t e2m1x8_from_quotients(const float (&q)[8]) {
 // (Markstein's division theorem; s has a 4-bit significand, far from the one excluded divisor),
 // i.e. the same bits as the division. Quotients so small that they
 // leave the normal range encode as 0 whatever their last bit is; the only thing that depends on
-// them is the sign bit of a negative value whose quotient rounds to zero, which needs |x| below
-// 2^-141 and is sent through the real division (FP32 input only: no bf16 or fp16 value is that
-// small).
-template <bool TINY_POSSIBLE>
+// them is the sign bit, (q < 0): it is clear where the quotient rounds to zero, which is where
+// |x| <= s * 2^-150 (the tie goes to the even zero). Both sides times 2^100 are exact, so one product
+// and one compare decide it, for -0.0 too.
 __device__ __forceinline__ uint32_t quantise_block(const float (&v)[16], uint2& packed) {
     uint32_t mx = 0;
     #pragma unroll
@@ -80,6 +79,7 @@ __device__ __forceinline__ uint32_t quantise_block(const float (&v)[16], uint2& 
     // Magnitudes are clamped to 8 * s: everything above 5 * s encodes as 6 anyway, and the clamp
     // keeps the product finite when the scale saturated at 448 or sits in the E4M3 subnormals.
     const float limit = 8.0f * s;
+    const float below = s * -0x1p-50f;
     uint32_t words[2];
     #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -92,9 +92,7 @@ __device__ __forceinline__ uint32_t quantise_block(const float (&v)[16], uint2& 
             const float q0 = __fmul_rn(ax, r);
             const float e = __fmaf_rn(-q0, s, ax);
             q[i] = __fmaf_rn(e, r, q0);
-            bool negative = x < 0.0f;
-            if (TINY_POSSIBLE && ax < 1e-42f) negative = negative && __fdiv_rn(ax, s) != 0.0f;
-            signs |= negative ? (8u << (4 * i)) : 0u;
+            signs |= __fmul_rn(x, 0x1p100f) < below ? (8u << (4 * i)) : 0u;
         }
         words[h] = e2m1x8_from_quotients(q) | signs;
     }

@@ -251,3 +251,18 @@ def test_two_level_scaling_is_bit_exact_and_recovers_the_product(g, dtype):
     # without the tensor scale the small operand loses its block scales to the E4M3 subnormals
     _, s_plain = g.quantize(b)
     assert int(to_np(s_plain).max()) < int(to_np(sb).max())
+
+
+def test_signs_of_quotients_at_the_edge_of_zero(g):
+    # FP32: the sign bit is (x / s < 0), clear where the quotient rounds to zero: |x| <= s * 2^-150, the tie included.
+    # Every multiple of the smallest subnormal around that edge, for scales from the smallest to 448, and -0.0.
+    rows = []
+    for amax in (0.0, 0.01, 0.3, 6.0, 40.0, 700.0, 2688.0, 1e6):
+        for first in range(0, 900, 15):
+            bits = np.arange(first, first + 15, dtype=np.uint32) | np.uint32(0x80000000)
+            rows.append(np.concatenate((bits.view(np.float32), np.array([amax], np.float32))))
+    x = np.stack(rows).astype(np.float32)
+    x = np.concatenate((x, -x)).reshape(-1, 64)
+    packed, scales = g.quantize(torch.from_numpy(x).cuda())
+    want, want_scales = O.quantize_padded(x)
+    assert np.array_equal(packed.cpu().numpy(), want) and np.array_equal(scales.cpu().numpy(), want_scales)
