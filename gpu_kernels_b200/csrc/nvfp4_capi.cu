@@ -559,6 +559,13 @@ int gpu_kernels_nvfp4_grouped_set_valid_rows(void* plan, const void* block_valid
     });
 }
 
+int gpu_kernels_nvfp4_grouped_set_static_weights(void* plan, int on) {
+    return guarded([&] {
+        if (!plan) throw std::invalid_argument("grouped set_static_weights: null plan");
+        static_cast<nvfp4_b200::GroupedGemm*>(plan)->static_weights = on ? 1 : 0;
+    });
+}
+
 int gpu_kernels_nvfp4_grouped_run(void* plan, void* C, int out_bf16, void* stream) {
     return guarded([&] {
         if (!plan) throw std::invalid_argument("null plan");

@@ -215,6 +215,9 @@ struct GemmArgs {
     // stages of B are requested before the wait; 2 = none of the operands: only the epilogue waits, before its
     // first store, so the tiles of this launch run while the tail of the previous one drains.
     int static_operands;
+    // 1: the kernel behind this one may start only once the grid in front of this one has finished (the trigger comes
+    // after the wait instead of before it). With it that kernel may rely on everything older than this launch.
+    int late_trigger;
     // EPI_DIRECT_RAGGED (one tile row, M = 128): the N columns are dealt to exactly as many tiles as there are
     // SMs, in units of 64 columns: the first ragged_extra tiles are ragged_base + 1 units wide, the others
     // ragged_base (2 or 3), so that no SM is left without a tile when N / 256 is smaller than the SM count. B is
@@ -290,7 +293,8 @@ __device__ __forceinline__ void tile_coords(int t, const GemmArgs& g, int& tm, i
         // grouped: all N tiles of one row block are consecutive, so an expert's weights are streamed once
         tm = t / g.tiles_n;
         tn = t - tm * g.tiles_n;
-        b_base = __ldg(g.block_expert + tm) * g.b_rows_per_expert;
+        // past L1: under static_operands it is read before the wait, when another batch's table may still be cached there
+        b_base = __ldcg(g.block_expert + tm) * g.b_rows_per_expert;
         return;
     }
     b_base = 0;
@@ -744,7 +748,10 @@ struct Roles {
         long long wait_acc = 0, wait_store = 0;
         const long long born = now();
         // with static operands the prologue did not wait for the grid in front: nothing may be stored before it has finished
-        if (g.static_operands != 0) grid_dependency_wait();
+        if (g.static_operands != 0) {
+            grid_dependency_wait();
+            if (g.late_trigger && threadIdx.x == 0) grid_launch_dependents();
+        }
         Walk walk(g, unit, units, tiles, g.ksteps);
         Segment seg;
         constexpr uint32_t SK_WARP_FLOATS = UN * 32;            // one warp's 32 rows of a tile
@@ -953,7 +960,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     // Programmatic dependent launch: a kernel launched behind this one with the stream-serialisation attribute
     // may bring its CTAs onto SMs that are free (and set up its barriers and Tensor Memory there) as soon as every
     // CTA of this grid has got here; it then waits in grid_dependency_wait() until this grid has finished.
-    if (threadIdx.x == 0) grid_launch_dependents();
+    if (threadIdx.x == 0 && !g.late_trigger) grid_launch_dependents();
     if (PROF && threadIdx.x == 0) g.prof[(size_t(CG == 2 ? blockIdx.x / 2u : blockIdx.x) * CG + rank) * PROF_WORDS + PROF_T_ENTER] = globaltimer_ns();
 
     if (threadIdx.x == 0) {
@@ -989,10 +996,13 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     // Everything above touched only this CTA's own resources. From here on global memory is read and written:
     // wait for the grid this launch depends on (returns at once when the launch was an ordinary one), unless the
     // caller has declared operands that the grid in front cannot be writing (then the roles wait where they must).
-    if (g.static_operands == 0) grid_dependency_wait();
+    if (g.static_operands == 0) {
+        grid_dependency_wait();
+        if (g.late_trigger && threadIdx.x == 0) grid_launch_dependents();
+    }
 
     Roles<CG, UN, EPI, PROF, MX> roles{smem, ctrl, rank, unit, gridDim.x / CG,
-                                   uint32_t(g.block_expert ? __ldg(g.num_blocks) : g.tiles_m) * uint32_t(g.tiles_n),
+                                   uint32_t(g.block_expert ? __ldcg(g.num_blocks) : g.tiles_m) * uint32_t(g.tiles_n),
                                    CG == 2 ? map_to_cta(smem_u32(const_cast<uint32_t*>(&ctrl->wait.abort)), rank ^ 1u) : 0u, g};
 
     if (warp == 5) {
@@ -1583,6 +1593,7 @@ void grouped_prepare(GroupedGemm& p, const uint8_t* A, const uint8_t* B, const u
                      int pool_rows, int n, int k, int experts, int block_rows, const int* block_expert,
                      const int* num_blocks) {
     p.block_valid = nullptr;
+    p.static_weights = 0;
     require_sm100();
     if (block_rows != 128 && block_rows != 256) throw std::invalid_argument("grouped gemm: block rows must be 128 or 256");
     if (pool_rows <= 0 || pool_rows % block_rows) throw std::invalid_argument("grouped gemm: pool rows must be a positive multiple of the block rows");
@@ -1644,6 +1655,7 @@ void grouped_launch_fused(const GroupedGemm& p, void* C, int out_bf16, uint8_t* 
     g.act_scales = act_scales;
     g.row_weight = row_weight;
     g.swiglu_clamp = clamp;
+    g.static_operands = g.late_trigger = row_dst ? 0 : p.static_weights;
     g.row_dst = row_dst;
     g.slots = slots;
     g.world = world;

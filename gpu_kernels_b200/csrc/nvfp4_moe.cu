@@ -492,7 +492,9 @@ quantise_route_kernel(const __nv_bfloat16* __restrict__ x, const long long* __re
                       int* __restrict__ error,
                       uint8_t* __restrict__ pool_packed, uint8_t* __restrict__ pool_scales,
                       float* __restrict__ pool_weight, int* __restrict__ route_row) {
-    chain_point();
+    // the wait before the trigger: the first expert GEMM behind this kernel reads the routing plan before its own wait
+    ptx::grid_dependency_wait();
+    ptx::grid_launch_dependents();
     extern __shared__ __align__(16) uint8_t smem_rows[];        // ROUTE_BUFFERS x (codes [hidden/2] | scale bytes [hidden/16] | int dst[topk])
     const int row_bytes = hidden / 2 + hidden / 16;
     const int dst_off = (row_bytes + 15) & ~15;

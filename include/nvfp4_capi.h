@@ -186,6 +186,11 @@ void gpu_kernels_nvfp4_grouped_plan_destroy(void* plan);
  * writes only the real rows of C: the padding rows of a pool of 128- or 256-row blocks (most of the pool when an
  * expert sees a few rows) stay out of HBM, and the caller must not read them. */
 int gpu_kernels_nvfp4_grouped_set_valid_rows(void* plan, const void* block_valid);
+/* on = 1: the caller promises that B, its scales, block_expert and num_blocks are complete once the grid in front of the
+ * kernel in front of each launch has finished, and that this kernel triggers its dependents only after its own wait (the
+ * dispatch kernel does, and a grouped launch with this option does). The launch then requests its first weight tiles
+ * while that kernel runs. 0 (default): nothing is read before the wait. Ignored by gpu_kernels_nvfp4_grouped_run_scatter. */
+int gpu_kernels_nvfp4_grouped_set_static_weights(void* plan, int on);
 int gpu_kernels_nvfp4_grouped_run(void* plan, void* C, int out_bf16, void* stream);
 
 /* The first expert GEMM with the activation fused into its epilogue (FC1 + kernels/moe/swiglu.cu:12-26 + the
