@@ -9,6 +9,8 @@ from __future__ import annotations
 import ctypes
 from pathlib import Path
 
+import torch
+
 P, I, F = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
 
 ROOT = Path(__file__).resolve().parents[1]
@@ -99,6 +101,28 @@ def load() -> ctypes.CDLL:
 def check(status: int) -> None:
     if status:
         raise Nvfp4Error(load().gpu_kernels_nvfp4_last_error().decode())
+
+
+def stream() -> int:
+    """Handle of the current device's current stream. torch.cuda.current_stream() builds a Stream object around it,
+    which took as long as the rest of a call's checks."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+class _Here:
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_HERE = _Here()
+
+
+def on(device: torch.device):
+    """Context in which `device` is the current one: nothing to do where it already is."""
+    return _HERE if device.index == torch._C._cuda_getDevice() else torch.cuda.device(device)
 
 
 def launch_count() -> int:

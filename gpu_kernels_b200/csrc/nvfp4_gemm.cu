@@ -1488,7 +1488,8 @@ void launch_with(const gpu_kernels::Nvfp4Params& p, void* C, cudaStream_t stream
     if (prof && (p.split_k > 1 || p.gather_world)) throw std::invalid_argument("nvfp4 gemm profile: plain plans only");
     if ((reinterpret_cast<uintptr_t>(C) & 31) && (p.split_k > 1 || (prof && p.direct_store)))
         throw std::invalid_argument("nvfp4 gemm: split-K and profiled launches store 32 bytes at a time: C must be 32-byte aligned");
-    const CUtensorMap tmC = output_map(C, p.M, p.N, p.out_bf16 != 0);
+    // only the staged route stores C through a map
+    const CUtensorMap tmC = p.direct_store ? CUtensorMap{} : output_map(C, p.M, p.N, p.out_bf16 != 0);
     const GemmArgs g = dense_args(p, C, prof);
     if (p.plain_tile_n && p.split_k <= 1 && !p.gather_world && !p.ragged_units && !p.route && p.direct_store && !prof) {
         if (p.plain_cta_group == 2) launch_plain<2, 256>(p, tmC, g, stream);
@@ -1631,8 +1632,7 @@ void grouped_launch_fused(const GroupedGemm& p, void* C, int out_bf16, uint8_t* 
     }
     if (fused && (!act_scales || !row_weight)) throw std::invalid_argument("grouped gemm: fused SwiGLU needs scales and row weights");
     if (!fused && (!C || (reinterpret_cast<uintptr_t>(C) & 15))) throw std::invalid_argument("grouped gemm: C must be 16-byte aligned");
-    if (fused) C = act_packed;       // only the tensor map needs a valid address; the fused route never stores C
-    const CUtensorMap tmC = output_map(C, p.pool_rows, p.n, out_bf16 != 0);
+    const CUtensorMap tmC{};         // no grouped route stores C through a map
     GemmArgs g{};
     g.M = p.pool_rows; g.N = p.n; g.K = p.k;
     g.ksteps = (p.k + STAGE_K - 1) / STAGE_K;

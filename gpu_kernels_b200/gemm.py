@@ -15,10 +15,6 @@ import torch
 from . import _lib
 
 
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
-
-
 class Nvfp4Gemm:
     def __init__(self, a_packed, b_packed, sfa, sfb, alpha: float = 1.0, workspace: torch.Tensor | None = None,
                  mx: bool = False):
@@ -41,17 +37,17 @@ class Nvfp4Gemm:
         self.out_dtype = torch.float16
         self._plan = ctypes.c_void_p()
         lib = _lib.load()
-        with torch.cuda.device(self.device):
+        with _lib.on(self.device):
             if mx:
                 _lib.check(lib.gpu_kernels_nvfp4_plan_create_mx(
                     ctypes.byref(self._plan), self.m, self.n, self.k, a_packed.data_ptr(), b_packed.data_ptr(),
-                    sfa.data_ptr(), sfb.data_ptr(), _stream()))
+                    sfa.data_ptr(), sfb.data_ptr(), _lib.stream()))
             else:
                 _lib.check(lib.gpu_kernels_nvfp4_plan_create(
                     ctypes.byref(self._plan), self.m, self.n, self.k, a_packed.data_ptr(), b_packed.data_ptr(),
                     sfa.data_ptr(), sfb.data_ptr(),
                     workspace.data_ptr() if workspace is not None else None,
-                    workspace.numel() if workspace is not None else 0, _stream()))
+                    workspace.numel() if workspace is not None else 0, _lib.stream()))
         if alpha != 1.0:
             self.set_alpha(alpha)
 
@@ -60,7 +56,7 @@ class Nvfp4Gemm:
 
     def set_option(self, key: str, value: int) -> None:
         # some options allocate or launch (split_k, l2_side): on the plan's own device
-        with torch.cuda.device(self.device):
+        with _lib.on(self.device):
             _lib.check(_lib.load().gpu_kernels_nvfp4_plan_set_option(self._plan, key.encode(), int(value)))
         if key == "out_bf16":
             self.out_dtype = torch.bfloat16 if value else torch.float16
@@ -75,7 +71,7 @@ class Nvfp4Gemm:
     def placement_misses(self) -> int:
         """Clusters (summed over launches) that ran on the other L2 side than the tile route assumed."""
         n = ctypes.c_uint()
-        with torch.cuda.device(self.device):
+        with _lib.on(self.device):
             _lib.check(_lib.load().gpu_kernels_nvfp4_plan_placement_misses(self._plan, ctypes.byref(n)))
         return int(n.value)
 
@@ -84,8 +80,8 @@ class Nvfp4Gemm:
             out = torch.empty((self.m, self.n), dtype=self.out_dtype, device=self.device)
         if not (out.is_cuda and out.dtype == self.out_dtype and out.is_contiguous() and out.shape == (self.m, self.n)):
             raise ValueError(f"out must be a contiguous CUDA {self.out_dtype} tensor [M, N]")
-        with torch.cuda.device(self.device):
-            _lib.check(_lib.load().gpu_kernels_nvfp4_custom(self._plan, out.data_ptr(), _stream()))
+        with _lib.on(self.device):
+            _lib.check(_lib.load().gpu_kernels_nvfp4_custom(self._plan, out.data_ptr(), _lib.stream()))
         return out
 
     def linear(self, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
@@ -98,8 +94,8 @@ class Nvfp4Gemm:
             raise ValueError("linear: NVFP4 plans only")
         if out is None:
             out = torch.empty((self.m, self.n), dtype=self.out_dtype, device=self.device)
-        with torch.cuda.device(self.device):
-            _lib.check(_lib.load().gpu_kernels_nvfp4_linear(self._plan, x.data_ptr(), _DTYPES[x.dtype], out.data_ptr(), _stream()))
+        with _lib.on(self.device):
+            _lib.check(_lib.load().gpu_kernels_nvfp4_linear(self._plan, x.data_ptr(), _DTYPES[x.dtype], out.data_ptr(), _lib.stream()))
         return out
 
     def profile(self, out: torch.Tensor):
@@ -107,8 +103,8 @@ class Nvfp4Gemm:
         n = 4096 * 16
         buf = (ctypes.c_ulonglong * n)()
         written = ctypes.c_int()
-        with torch.cuda.device(self.device):
-            _lib.check(_lib.load().gpu_kernels_nvfp4_plan_profile(self._plan, out.data_ptr(), _stream(), buf, n,
+        with _lib.on(self.device):
+            _lib.check(_lib.load().gpu_kernels_nvfp4_plan_profile(self._plan, out.data_ptr(), _lib.stream(), buf, n,
                                                                   ctypes.byref(written)))
         keys = ("producer_wait", "producer_total", "mma_wait_data", "mma_wait_acc", "mma_total",
                 "epi_wait_acc", "epi_wait_store", "epi_total", "smid",
@@ -121,12 +117,12 @@ class Nvfp4Gemm:
     def run_cublaslt(self, out: torch.Tensor) -> torch.Tensor:
         """cuBLASLt's NVFP4 matmul on the same operands (comparison only)."""
         a, b = self._keep[0], self._keep[1]
-        with torch.cuda.device(self.device):
-            _lib.check(_lib.load().gpu_kernels_nvfp4_cublas(self._plan, out.data_ptr(), a.data_ptr(), b.data_ptr(), _stream()))
+        with _lib.on(self.device):
+            _lib.check(_lib.load().gpu_kernels_nvfp4_cublas(self._plan, out.data_ptr(), a.data_ptr(), b.data_ptr(), _lib.stream()))
         return out
 
     def validate(self) -> None:
-        with torch.cuda.device(self.device):
+        with _lib.on(self.device):
             _lib.check(_lib.load().gpu_kernels_nvfp4_validate(self._plan))
 
     def close(self) -> None:
@@ -150,7 +146,7 @@ def gemm_host(a_packed, b_packed, sfa, sfb, out, alpha: float = 1.0) -> torch.Te
     n = b_packed.shape[0]
     _lib.check(_lib.load().gpu_kernels_nvfp4_gemm_host(
         m, n, 2 * half_k, a_packed.data_ptr(), b_packed.data_ptr(), sfa.data_ptr(), sfb.data_ptr(),
-        out.data_ptr(), float(alpha), _stream()))
+        out.data_ptr(), float(alpha), _lib.stream()))
     return out
 
 

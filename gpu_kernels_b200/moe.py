@@ -23,10 +23,6 @@ from .peer import DeviceView, PeerGroup, SharedBuffer
 from .nvfp4 import quantize
 
 
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
-
-
 def exchange_splits(counts_matrix: torch.Tensor, rank: int, local_experts: int, block_rows: int = 128):
     """Row counts of the two all-to-alls from the all-gathered route counts.
 
@@ -225,7 +221,7 @@ class Nvfp4MoE:
 
     # ---- phases ----------------------------------------------------------------------------------
     def _metadata(self, ids, tokens, block_rows):
-        lib, s = _lib.load(), _stream()
+        lib, s = _lib.load(), _lib.stream()
         routes = tokens * self.topk
         if self.world == 1 and routes <= 32768:
             # one launch: histogram of the routes (by the plan's single CTA: 24576 routes take it less time than
@@ -289,7 +285,7 @@ class Nvfp4MoE:
         ids = ids.contiguous().to(torch.int64)
         weights = weights.contiguous().to(torch.float32)
         with torch.cuda.device(self.device):
-            s = _stream()
+            s = _lib.stream()
             fused_dispatch = self.fused_dispatch and (self.world == 1 or self._peer is not None)
             self._mark("start")
             if not fused_dispatch:

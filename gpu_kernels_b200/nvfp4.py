@@ -9,15 +9,12 @@ are rejected.
 """
 from __future__ import annotations
 
+import numpy as np
 import torch
 
 from . import _lib
 
 _DTYPES = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
-
-
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
 
 
 def scale_rows(rows: int) -> int:
@@ -47,20 +44,21 @@ def quantize(values: torch.Tensor, tensor_scale: float | None = None):
     rows, k = values.shape
     packed = torch.empty((rows, k // 2), dtype=torch.uint8, device=values.device)
     scales = torch.empty((scale_rows(rows) * k // 16,), dtype=torch.uint8, device=values.device)
-    with torch.cuda.device(values.device):
+    with _lib.on(values.device):
         if tensor_scale is None:
             _lib.check(_lib.load().gpu_kernels_nvfp4_quantize(
-                values.data_ptr(), _DTYPES[values.dtype], packed.data_ptr(), scales.data_ptr(), rows, k, _stream()))
+                values.data_ptr(), _DTYPES[values.dtype], packed.data_ptr(), scales.data_ptr(), rows, k, _lib.stream()))
         else:
             _lib.check(_lib.load().gpu_kernels_nvfp4_quantize_scaled(
                 values.data_ptr(), _DTYPES[values.dtype], inverse_tensor_scale(tensor_scale), packed.data_ptr(),
-                scales.data_ptr(), rows, k, _stream()))
+                scales.data_ptr(), rows, k, _lib.stream()))
     return packed, scales
 
 
 def inverse_tensor_scale(tensor_scale: float) -> float:
     """float32(1 / tensor_scale) as a Python float: the multiplier the scaled quantiser applies."""
-    return float(torch.tensor(1.0, dtype=torch.float32) / torch.tensor(float(tensor_scale), dtype=torch.float32))
+    with np.errstate(all="ignore"):
+        return float(np.float32(1.0) / np.float32(tensor_scale))
 
 
 def tensor_scale_for(values: torch.Tensor) -> float:
@@ -78,9 +76,9 @@ def dequantize(packed: torch.Tensor, scales: torch.Tensor) -> torch.Tensor:
     if scales.numel() != scale_rows(rows) * half_k // 8:
         raise ValueError("scales must hold ceil(rows/128)*128*K/16 bytes")
     out = torch.empty((rows, 2 * half_k), dtype=torch.float32, device=packed.device)
-    with torch.cuda.device(packed.device):
+    with _lib.on(packed.device):
         _lib.check(_lib.load().gpu_kernels_nvfp4_dequantize(
-            packed.data_ptr(), scales.data_ptr(), out.data_ptr(), rows, 2 * half_k, _stream()))
+            packed.data_ptr(), scales.data_ptr(), out.data_ptr(), rows, 2 * half_k, _lib.stream()))
     return out
 
 
@@ -110,9 +108,9 @@ def quantize_mx(values: torch.Tensor):
     rows, k = values.shape
     packed = torch.empty((rows, k // 2), dtype=torch.uint8, device=values.device)
     scales = torch.empty((scale_rows(rows) * k // 32,), dtype=torch.uint8, device=values.device)
-    with torch.cuda.device(values.device):
+    with _lib.on(values.device):
         _lib.check(_lib.load().gpu_kernels_nvfp4_quantize_mx(
-            values.data_ptr(), _DTYPES[values.dtype], packed.data_ptr(), scales.data_ptr(), rows, k, _stream()))
+            values.data_ptr(), _DTYPES[values.dtype], packed.data_ptr(), scales.data_ptr(), rows, k, _lib.stream()))
     return packed, scales
 
 
@@ -125,7 +123,7 @@ def dequantize_mx(packed: torch.Tensor, scales: torch.Tensor) -> torch.Tensor:
     if scales.numel() != scale_rows(rows) * half_k // 16:
         raise ValueError("scales must hold ceil(rows/128)*128*K/32 bytes")
     out = torch.empty((rows, 2 * half_k), dtype=torch.float32, device=packed.device)
-    with torch.cuda.device(packed.device):
+    with _lib.on(packed.device):
         _lib.check(_lib.load().gpu_kernels_nvfp4_dequantize_mx(
-            packed.data_ptr(), scales.data_ptr(), out.data_ptr(), rows, 2 * half_k, _stream()))
+            packed.data_ptr(), scales.data_ptr(), out.data_ptr(), rows, 2 * half_k, _lib.stream()))
     return out
