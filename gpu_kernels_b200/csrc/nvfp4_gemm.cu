@@ -69,7 +69,8 @@ enum Epi : int {
     EPI_GATHER_DIRECT = 6, // the same with register stores
     EPI_SPLIT_K = 7,       // FP32 partial sums + finish (to C or to every rank's full C)
     EPI_DIRECT_RAGGED = 8, // EPI_DIRECT on single-CTA tiles of unequal width (see GemmArgs::ragged_base)
-    EPI_DIRECT_EDGE = 9,   // EPI_DIRECT with rows >= M and columns >= N masked (M, N not multiples of the tile), 16-byte stores
+    EPI_DIRECT_EDGE = 9,   // EPI_DIRECT with rows >= M and columns >= N masked (M, N not multiples of the tile)
+    EPI_DIRECT_TWIN = 10,  // EPI_DIRECT_EDGE on narrow tiles, one per CTA, with two issuers and two producers (see TWIN)
 };
 
 // MX: the MXFP4 flavour of the same instruction: one UE8M0 (power-of-two) scale per 32 values, so a 512-byte
@@ -106,10 +107,18 @@ struct Config {
     // launch with one tile per CTA. The routes that stage in shared memory keep one warp per quarter (a second
     // set of staging buffers would cost a ring stage), as does split-K.
     static constexpr int EPI_WARPS = (EPI == EPI_DIRECT || EPI == EPI_ACT || EPI == EPI_SCATTER || EPI == EPI_GATHER_DIRECT ||
-                                      EPI == EPI_DIRECT_RAGGED || EPI == EPI_DIRECT_EDGE) ? 8 : 4;
+                                      EPI == EPI_DIRECT_RAGGED || EPI == EPI_DIRECT_EDGE || EPI == EPI_DIRECT_TWIN) ? 8 : 4;
+    static constexpr bool MASKED = EPI == EPI_DIRECT_EDGE || EPI == EPI_DIRECT_TWIN;
+    // Two issuers and two producers, each with every other ring step, into an accumulator and scale columns of their
+    // own; the epilogue adds the two. What bounds a narrow tile is neither memory nor the tensor pipe but the
+    // instructions of one step: stamps of a 128 x 128 tile gave the issuer 450 cycles for eight scale copies, four MMAs
+    // and the commit, the producer 230 for four requests and 300 for its loop, and the same time per step with the
+    // MMAs, the copies or the scale requests left out.
+    static constexpr bool TWIN = EPI == EPI_DIRECT_TWIN;
+    static_assert(!TWIN || (CG == 1 && UN <= 128), "two accumulators and two sets of scale columns in Tensor Memory");
     static constexpr bool RAGGED = EPI == EPI_DIRECT_RAGGED;
     static_assert(!RAGGED || (CG == 1 && UN == 256), "ragged tiles are single-CTA tiles of up to 256 columns");
-    static constexpr int THREADS = (2 + EPI_WARPS) * 32;        // warps 0-3 epilogue, 4 MMA, 5 producer, 6-9 epilogue
+    static constexpr int THREADS = ((TWIN ? 4 : 2) + EPI_WARPS) * 32;        // warps 0-3 epilogue, 4 MMA, 5 producer, 6-9 epilogue, 10 MMA, 11 producer
     static constexpr int ROW_PITCH = UN * 2 + 16;
     static constexpr int EPI_BYTES = ROW_STAGING ? 4 * 32 * ROW_PITCH : STAGED_EPILOGUE ? 4 * 2 * EPI_WARP_BYTES : 0;
     static constexpr int CTRL_BYTES = 1024;
@@ -125,6 +134,7 @@ struct Config {
     static_assert(OVERLAP <= EPI_COLS, "the first epilogue chunk must cover the overlap");
     static_assert(STAGE_BYTES % 1024 == 0, "stages keep the 1024-byte swizzle alignment");
     static_assert(STAGES >= 3 && STAGES <= 8, "ring depth");
+    static_assert(!TWIN || (STAGES % 2 == 0 && 2 * UN + 2 * SF_COLS <= TMEM_COLS), "every other ring stage is one issuer's");
     static_assert(!STAGED_EPILOGUE || CG == 2, "single CTAs write C from registers");
     // Instruction descriptor of kind::mxf4nvf4: A and B E2M1 (format 1) at bits 7 and 10,
     // both K-major, N >> 3 at bit 17, UE4M3 scales (bit 23 = 0), M >> 4 at bit 24,
@@ -336,7 +346,7 @@ struct Roles {
     // atoms of a K = 256 step, and a last partial step reads zeros beyond the block's own atoms (as the
     // operand maps do beyond K/2 bytes), so K only has to be a multiple of 64.
     __device__ void produce(const CUtensorMap* tmA, const CUtensorMap* tmB,
-                            const CUtensorMap* tmSFA, const CUtensorMap* tmSFB, int lane) const {
+                            const CUtensorMap* tmSFA, const CUtensorMap* tmSFB, int lane, int who = 0) const {
         int stage = 0;
         uint32_t phase = 0;
         const int ksteps = g.ksteps;
@@ -363,7 +373,7 @@ struct Roles {
             // copy unit longer than one it has to fetch (about 6 cycles a row).
             bool b_live = true;
             int sfb_live = Cfg::SFB_BLOCKS;
-            if constexpr (EPI == EPI_DIRECT_EDGE) {
+            if constexpr (Cfg::MASKED) {
                 if (!g.block_expert) {
                     const int blocks = (g.N + 127) / 128;
                     b_live = b_row < g.N;
@@ -380,8 +390,8 @@ struct Roles {
             } else {
                 stage_bytes = CG * Cfg::STAGE_BYTES;
             }
-            const bool a_live = EPI != EPI_DIRECT_EDGE || CG == 1 || a_row < g.M;
-            const bool whole = EPI != EPI_DIRECT_EDGE || (a_live && b_live && sfb_live == Cfg::SFB_BLOCKS);
+            const bool a_live = !Cfg::MASKED || CG == 1 || a_row < g.M;
+            const bool whole = !Cfg::MASKED || (a_live && b_live && sfb_live == Cfg::SFB_BLOCKS);
             if constexpr (Cfg::RAGGED) {
                 int n0, width;
                 ragged_span(g, tn, n0, width);
@@ -397,6 +407,12 @@ struct Roles {
             const int k_first = (g.k_skew && g.split_k <= 1) ? int((place * uint32_t(g.k_skew)) % uint32_t(ksteps)) : 0;
             for (int step = seg.k0; step < seg.k1; ++step) {
                 const int ks = step + k_first < ksteps ? step + k_first : step + k_first - ksteps;
+                if (Cfg::TWIN && (issued & 1) != who) {         // the other producer's step
+                    ++issued;
+                    if (early_b && issued == Cfg::STAGES) release_held(tmA, tmSFA, held, Cfg::STAGES, who);
+                    if (++stage == Cfg::STAGES) { stage = 0; phase ^= 1u; }
+                    continue;
+                }
                 const long long w0 = now();
                 const bool ok = wait(&ctrl->empty[stage], phase ^ 1u, lane == 0 ? STATUS_TIMEOUT_PRODUCER : 0u,
                                      0x10000000u | (stage << 16) | ks);
@@ -449,11 +465,11 @@ struct Roles {
                     }
                 }
                 ++issued;
-                if (early_b && issued == Cfg::STAGES) release_held(tmA, tmSFA, held, Cfg::STAGES);
+                if (early_b && issued == Cfg::STAGES) release_held(tmA, tmSFA, held, Cfg::STAGES, who);
                 if (++stage == Cfg::STAGES) { stage = 0; phase ^= 1u; }
             }
         }
-        if (early_b && issued < Cfg::STAGES) release_held(tmA, tmSFA, held, issued);   // fewer steps than ring stages
+        if (early_b && issued < Cfg::STAGES) release_held(tmA, tmSFA, held, issued, who);   // fewer steps than ring stages
         if (PROF && lane == 0) {
             unsigned long long* out = g.prof + (size_t(unit) * CG + rank) * PROF_WORDS;
             out[PROF_PROD_WAIT] = waited;
@@ -464,10 +480,10 @@ struct Roles {
     // The A halves (rows of A and their scale atoms) of the first `count` ring stages, once the grid this launch
     // depends on has finished: stage i of the ring, in issue order.
     struct Held { int ks, a_row, sfa_block; };
-    __device__ void release_held(const CUtensorMap* tmA, const CUtensorMap* tmSFA, const Held* held, int count) const {
+    __device__ void release_held(const CUtensorMap* tmA, const CUtensorMap* tmSFA, const Held* held, int count, int who) const {
         grid_dependency_wait();
         if (elect_one()) {
-            for (int i = 0; i < count; ++i) {
+            for (int i = Cfg::TWIN ? who : 0; i < count; i += Cfg::TWIN ? 2 : 1) {
                 const uint32_t base = smem + i * Cfg::STAGE_BYTES;
                 const uint32_t own_full = bar(&ctrl->full[i]);
                 if constexpr (CG == 1) {
@@ -490,8 +506,9 @@ struct Roles {
     // before this stage's instructions are issued, so its latency hides behind them and the
     // blocking wait is skipped when the probe succeeded; and every descriptor is a uniform
     // 32-bit add on values computed outside the one-lane block.
-    __device__ void issue(uint32_t tmem, int lane) const {
-        int stage = 0;
+    __device__ void issue(uint32_t tmem, int lane, int who = 0) const {
+        constexpr int STRIDE = Cfg::TWIN ? 2 : 1;
+        int stage = who;
         uint32_t phase = 0, iter = 0;
         const int ksteps = g.ksteps;
         long long wait_full = 0, wait_acc = 0;
@@ -502,12 +519,12 @@ struct Roles {
         constexpr uint32_t SCALE_HI = (128u >> 4) | (1u << 14);
         constexpr uint32_t SCALE_LBO = (16u >> 4) << 16;
         const uint32_t ring_lo = (smem & 0x3FFFFu) >> 4;
-        const uint32_t sf_tmem = tmem + Cfg::SF_BASE;
+        const uint32_t sf_tmem = tmem + Cfg::SF_BASE - uint32_t(who) * Cfg::SF_COLS;
         bool landed = false;                                    // the probe of this step's barrier succeeded
         Walk walk(g, unit, units, tiles, ksteps);
         Segment seg;
         for (; walk.get(seg); ++iter) {
-            const uint32_t acc = tmem + (iter & 1u) * Cfg::ACC_STRIDE;
+            const uint32_t acc = tmem + (Cfg::TWIN ? uint32_t(who) : iter & 1u) * Cfg::ACC_STRIDE;
             uint32_t idesc = Cfg::IDESC, sfb_shift = 0;
             if constexpr (Cfg::RAGGED) {
                 int tm, tn, b_base, n0, width;
@@ -523,7 +540,7 @@ struct Roles {
             unsigned long long* tr = nullptr;
             if (PROF && unit == 0 && lane == 0 && iter > 0 && iter <= TR_TILES)
                 tr = g.prof + size_t(units) * CG * PROF_WORDS + size_t(iter - 1) * 8;
-            for (int ks = seg.k0; ks < seg.k1; ++ks) {
+            for (int ks = seg.k0 + who; ks < seg.k1; ks += STRIDE) {
                 if (!landed) {
                     const long long w0 = now();
                     const bool ok = wait(&ctrl->full[stage], phase, lane == 0 ? STATUS_TIMEOUT_MMA : 0u,
@@ -534,12 +551,12 @@ struct Roles {
                 if (PROF && iter == 0 && ks == seg.k0 && lane == 0)
                     g.prof[size_t(unit) * CG * PROF_WORDS + PROF_T_FIRST_DATA] = globaltimer_ns();
                 tc_fence_after_sync();
-                const int next_stage = stage + 1 == Cfg::STAGES ? 0 : stage + 1;
-                const uint32_t next_phase = stage + 1 == Cfg::STAGES ? phase ^ 1u : phase;
+                const int next_stage = stage + STRIDE >= Cfg::STAGES ? stage + STRIDE - Cfg::STAGES : stage + STRIDE;
+                const uint32_t next_phase = stage + STRIDE >= Cfg::STAGES ? phase ^ 1u : phase;
                 const bool probe = mbar_test_wait(bar(&ctrl->full[next_stage]), next_phase);
                 const uint32_t lo = ring_lo + uint32_t(stage) * (Cfg::STAGE_BYTES >> 4);
                 const uint32_t empty = bar(&ctrl->empty[stage]);
-                const uint32_t first = ks != seg.k0 ? 1u : 0u;   // 0: the first MMA of the segment overwrites the accumulator
+                const uint32_t first = ks != seg.k0 + who ? 1u : 0u;   // 0: the first MMA of the segment overwrites the accumulator
                 // j: the MMA (K = 64) inside the stage. NVFP4: MMA j has its own scale atom j. MXFP4: MMAs 2a and 2a+1
                 // share atom a (copied before the first of them) and read its bytes 0-1 and 2-3.
                 auto copies = [&](int j) {
@@ -562,7 +579,7 @@ struct Roles {
                                              OPERAND_HI, idesc | (sf_id << 29) | (sf_id << 4), sf, sf + 4 + sfb_shift,
                                              j != 0 ? 1u : first);
                 };
-                const bool handover = ks == seg.k0 && iter > 0;
+                const bool handover = !Cfg::TWIN && ks == seg.k0 && iter > 0;     // twins: one tile per CTA
                 if (handover) {
                     // First step of a tile: the scale copies do not touch the accumulators, so they go out
                     // before the wait for the epilogue to pull the columns this tile shares with the last one.
@@ -588,7 +605,7 @@ struct Roles {
                     #pragma unroll
                     for (int j = 0; j < STAGE_K / MMA_K; ++j) mma(j);
                     mma_commit<CG>(empty);                      // stage reusable once these MMAs retire
-                    if (ks == seg.k1 - 1) mma_commit<CG>(bar(&ctrl->acc_full));
+                    if (ks + STRIDE >= seg.k1) mma_commit<CG>(bar(&ctrl->acc_full));
                 }
                 if (tr && ks == seg.k0) tr[2] = now();
                 landed = __all_sync(0xFFFFFFFFu, probe);
@@ -762,7 +779,7 @@ struct Roles {
             const int row0 = tm * Cfg::TILE_M + int(rank) * BLOCK_M + warp * 32;
             int col0 = tn * UN, chunks = UN / EPI_COLS;
             int row_limit = g.M;                                 // EPI_DIRECT_EDGE: first row that is not written
-            if constexpr (EPI == EPI_DIRECT_EDGE || EPI == EPI_ACT) {
+            if constexpr (Cfg::MASKED || EPI == EPI_ACT) {
                 if (g.block_valid) row_limit = tm * Cfg::TILE_M + __ldg(g.block_valid + tm);
             }
             if constexpr (Cfg::RAGGED) {
@@ -797,6 +814,16 @@ struct Roles {
                 tmem_ld_32x32(acc + chunk * EPI_COLS, v);
                 tmem_ld_32x32(acc + chunk * EPI_COLS + 32, v + 32);
                 tmem_ld_wait();
+                if constexpr (Cfg::TWIN) {
+                    #pragma unroll
+                    for (int h = 0; h < EPI_COLS; h += 32) {
+                        uint32_t odd[32];
+                        tmem_ld_32x32(acc + Cfg::ACC_STRIDE + chunk * EPI_COLS + h, odd);
+                        tmem_ld_wait();
+                        #pragma unroll
+                        for (int i = 0; i < 32; ++i) v[h + i] = __float_as_uint(__uint_as_float(v[h + i]) + __uint_as_float(odd[i]));
+                    }
+                }
                 if (c == 0) {
                     if (tr && rank == 0) tr[1] = now();
                     tc_fence_before_sync();
@@ -887,7 +914,7 @@ struct Roles {
                                         v, alpha, true);
                 } else if constexpr (EPI == EPI_DIRECT || EPI == EPI_DIRECT_RAGGED) {
                     store_row_chunk(static_cast<uint16_t*>(g.c) + size_t(row0 + lane) * g.ldc + col0 + chunk * EPI_COLS, v, alpha, true);
-                } else if constexpr (EPI == EPI_DIRECT_EDGE) {
+                } else if constexpr (Cfg::MASKED) {
                     store_row_chunk_edge(static_cast<uint16_t*>(g.c) + size_t(row0 + lane) * g.ldc + col0 + chunk * EPI_COLS, v, alpha,
                                          row0 + lane < row_limit, g.N - (col0 + chunk * EPI_COLS));
                 } else {
@@ -944,7 +971,7 @@ struct Roles {
 };
 
 template <int CG, int UN, int EPI, bool PROF, bool MX = false>
-__global__ void __launch_bounds__(Config<CG, UN, EPI>::THREADS, 1)
+__global__ void __launch_bounds__(Config<CG, UN, EPI, MX>::THREADS, 1)
 nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                   const __grid_constant__ CUtensorMap tmSFA, const __grid_constant__ CUtensorMap tmSFB,
                   const __grid_constant__ CUtensorMap tmC, const GemmArgs g) {
@@ -968,7 +995,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             mbar_init(smem_u32(&ctrl->full[s]), 1);
             mbar_init(smem_u32(&ctrl->empty[s]), 1);
         }
-        mbar_init(smem_u32(&ctrl->acc_full), 1);
+        mbar_init(smem_u32(&ctrl->acc_full), Cfg::TWIN ? 2 : 1);
         mbar_init(smem_u32(&ctrl->acc_free), Cfg::EPI_WARPS * CG);   // one arrival per epilogue warp of the pair
         ctrl->wait.abort = 0;
         mbar_init_fence();
@@ -1009,6 +1036,10 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         roles.produce(&tmA, &tmB, &tmSFA, &tmSFB, lane);
     } else if (warp == 4) {
         if (rank == 0) roles.issue(tmem, lane);
+    } else if (Cfg::TWIN && warp == 10) {
+        roles.issue(tmem, lane, 1);
+    } else if (Cfg::TWIN && warp == 11) {
+        roles.produce(&tmA, &tmB, &tmSFA, &tmSFB, lane, 1);
     } else {
         roles.drain(tmem, &tmC, warp & 3, warp < 4 ? 0 : 1, lane);
     }
@@ -1202,7 +1233,7 @@ int band_rows(int units, int tiles_m) {
 //     last tile move half the bytes per FLOP.
 // Time estimate in ns: launch and first data, the exposed epilogue of the last tile, then a cost per ring step and
 // wave; fitted to M = 8..1024, N = 1536..28672, K = 2048..8192 within 10 %. At least as long as the weights need
-// from HBM. Measured (us, the plan's own tiles / these): 8 x 8192 x 8192 16.9 / 12.9, 128 x 4096 x 4096 11.5 / 8.0,
+// from HBM. Measured with one issuer (us, the plan's own tiles / these): 8 x 8192 x 8192 16.9 / 12.9, 128 x 4096 x 4096 11.5 / 8.0,
 // 512 x 2048 x 4096 10.0 / 8.2, 8 x 14336 x 4096 11.4 / 9.4, 4096 x 4224 x 4096 49.2 / 39.4, 4100 x 8320 x 4096
 // 103.6 / 83.0; where these would lose: 128 x 28672 x 8192 on 128-wide tiles 27.3 / 29.6.
 struct PlainTile { int cta_group, tile_n; float step_ns, tail_ns; };
@@ -1479,6 +1510,17 @@ void launch_plain(const gpu_kernels::Nvfp4Params& p, const CUtensorMap& tmC, con
     g.tiles_n = (p.N + UN - 1) / UN;
     g.group_m = p.plain_group_m;
     const bool pdl = p.pdl != 0;
+    if constexpr (CG == 1 && UN <= 128) {
+        // Twins: one tile per CTA, and a K loop long enough to pay for the larger block and the second accumulator.
+        // Measured (us, one issuer / two): 32 steps 8 x 8192 x 8192 12.8 / 11.5, 1 x 2048 x 8192 12.3 / 10.2; 28 steps
+        // 384 x 1536 x 7168 11.4 / 9.6; 16 steps 64 x 4096 x 4096 8.0 / 7.6, 8 x 14336 x 4096 9.5 / 9.5; 8 steps
+        // 300 x 2048 x 2048 5.7 / 6.0; 2 steps 1 x 4096 x 512 3.4 / 4.3.
+        if (g.tiles_m * g.tiles_n <= p.plain_units && g.ksteps >= 16) {
+            if (p.mx) launch_instance<1, UN, EPI_DIRECT_TWIN, false, true>(p.device, p.plain_units, p.A, p.plain_B, p.SFA, p.SFB, tmC, g, stream, pdl);
+            else launch_instance<1, UN, EPI_DIRECT_TWIN>(p.device, p.plain_units, p.A, p.plain_B, p.SFA, p.SFB, tmC, g, stream, pdl);
+            return;
+        }
+    }
     if (p.mx) launch_instance<CG, UN, EPI_DIRECT_EDGE, false, true>(p.device, p.plain_units, p.A, p.plain_B, p.SFA, p.SFB, tmC, g, stream, pdl);
     else launch_instance<CG, UN, EPI_DIRECT_EDGE>(p.device, p.plain_units, p.A, p.plain_B, p.SFA, p.SFB, tmC, g, stream, pdl);
 }

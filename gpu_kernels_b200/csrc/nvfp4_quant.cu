@@ -173,8 +173,9 @@ dequantise_kernel(const uint8_t* __restrict__ packed, const uint8_t* __restrict_
 // An all-zero block takes e = -127; a block with a NaN or an infinity takes the NaN scale 0xFF and the codes of
 // the NVFP4 NaN block. The scale bytes go to cuBLASLt's VEC32 order: the VEC16 atoms with K/32 blocks per row.
 // A CTA owns one scale atom, 128 rows x 128 columns: two blocks of 32 per thread, the second's loads in flight during the
-// first's arithmetic (16-bit inputs), the atom's bytes gathered in shared memory and written as one run (one thread per
-// block, each scale byte stored by itself: see the commit that replaced it for the figures).
+// first's arithmetic, the atom's bytes gathered in shared memory and written as one run. Against one thread per block with
+// each scale byte stored by itself: 8192 x 8192 bf16 39.4 -> 32.5 us (5.3 TB/s), 2048 x 2048 f16 4.8 -> 4.0 us; what
+// bounds it is HBM and the fixed cost of a launch, as for the NVFP4 kernel.
 template <typename T>
 __global__ void __launch_bounds__(Q_THREADS, sizeof(T) == 2 ? 4 : 3)
 quantise_mx_kernel(const T* __restrict__ x, uint8_t* __restrict__ packed, uint8_t* __restrict__ scales, int rows, int K) {

@@ -434,7 +434,7 @@ def test_m_and_n_that_are_not_whole_tiles(g, m, n, k, variant):
 # whose last tile has a half that lies wholly beyond N or M. (M, N, K, what the plan's own tiles are)
 PLAIN_TILE_SHAPES = [
     (1, 8, 64, 1064), (7, 136, 320, 1064), (129, 72, 512, 1064), (128, 192, 1088, 1064), (300, 1000, 2304, 1064),
-    (8, 8192, 2048, 1256), (512, 2048, 2048, 2256), (121, 3000, 1024, 1256), (1000, 4224, 1280, 1128), (300, 8192, 1536, 1256),
+    (8, 8192, 2048, 1256), (512, 2048, 2048, 2256), (5, 520, 4096, 1128), (130, 1000, 4416, 2256), (128, 14336, 4160, 1256), (121, 3000, 1024, 1256), (1000, 4224, 1280, 1128), (300, 8192, 1536, 1256),
     (1100, 4360, 1088, 1128),
 ]
 
@@ -497,6 +497,18 @@ def test_mxfp4_edge_shapes(g):
                O.dequantize_padded(to_np(pb), to_np(sb), O.dequantize_mx).T)
         assert_gemm_close(out, ref, f"mxfp4 edge {m}x{n}x{k}")
         plan.close()
+
+
+@pytest.mark.parametrize("m,n,k", [(7, 264, 4224), (128, 1536, 4096), (1, 8, 3968)])
+def test_mxfp4_narrow_tiles(g, m, n, k):
+    # few columns: 64-wide tiles with two issuers from 16 ring steps on, one below
+    pa, sa = g.quantize_mx(random_operand(m, k, seed=m + k))
+    pb, sb = g.quantize_mx(random_operand(n, k, seed=n + k, scale=0.05))
+    plan = g.Nvfp4Gemm(pa, pb, sa, sb, mx=True)
+    out = plan.run(torch.full((m, n), float("nan"), dtype=torch.float16, device="cuda"))
+    plan.validate()
+    assert_gemm_close(out, to_np(g.dequantize_mx(pa, sa) @ g.dequantize_mx(pb, sb).T), f"mxfp4 narrow {m}x{n}x{k}")
+    plan.close()
 
 
 def fp32_reference_on_gpu(g, pa, sa, pb, sb):
