@@ -1,6 +1,6 @@
 // NVFP4 block-scaled GEMM for B200 (sm_100a): C[M,N] fp16 = alpha * (A sfA)(B sfB)^T.
 //
-// One persistent kernel, three roles per CTA (192 or 320 threads):
+// One persistent kernel, three roles per CTA (192 or 320 threads; 384 where issuer and producer are doubled):
 //   warps 0-3  epilogue: TMEM -> registers -> FP16 -> swizzled shared memory -> TMA store, or straight to
 //              global memory (then warps 6-9 are a second set, two warps per Tensor Memory lane quarter)
 //   warp  4    MMA issuer (one elected lane): scale copies into TMEM + tcgen05 block-scaled MMAs
@@ -500,7 +500,7 @@ struct Roles {
 
     // ---- warp 4 of the leader CTA: scale copies and MMAs ------------------------------
     // Per ring step the warp spends its time on: noticing that the stage has landed, the 12
-    // scale copies + 4 MMAs + commit, and loop control. The tensor pipe needs 4 x 128 cycles per
+    // scale copies (8 on narrow tiles) + 4 MMAs + commit, and loop control. The tensor pipe needs 4 x 128 cycles per
     // step, so the thread side has to stay clearly below that or the pipe runs dry at every
     // step. Two things keep it there: the barrier of the NEXT stage is probed (non-blocking)
     // before this stage's instructions are issued, so its latency hides behind them and the
