@@ -501,7 +501,7 @@ def test_mxfp4_edge_shapes(g):
 
 @pytest.mark.parametrize("m,n,k", [(7, 264, 4224), (128, 1536, 4096), (1, 8, 3968)])
 def test_mxfp4_narrow_tiles(g, m, n, k):
-    # few columns: 64-wide tiles with two issuers from 16 ring steps on, one below
+    # few columns and 16 ring steps or more: 64-wide tiles with two issuers
     pa, sa = g.quantize_mx(random_operand(m, k, seed=m + k))
     pb, sb = g.quantize_mx(random_operand(n, k, seed=n + k, scale=0.05))
     plan = g.Nvfp4Gemm(pa, pb, sa, sb, mx=True)
