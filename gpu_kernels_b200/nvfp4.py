@@ -56,9 +56,10 @@ def quantize(values: torch.Tensor, tensor_scale: float | None = None):
 
 
 def inverse_tensor_scale(tensor_scale: float) -> float:
-    """float32(1 / tensor_scale) as a Python float: the multiplier the scaled quantiser applies."""
+    """float32(1 / tensor_scale) as a Python float: the multiplier the scaled quantiser applies. Anything float() takes,
+    a one-element tensor on any device included."""
     with np.errstate(all="ignore"):
-        return float(np.float32(1.0) / np.float32(tensor_scale))
+        return float(np.float32(1.0) / np.float32(float(tensor_scale)))
 
 
 def tensor_scale_for(values: torch.Tensor) -> float:
