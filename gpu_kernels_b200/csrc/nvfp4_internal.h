@@ -54,7 +54,10 @@ int l2_side_census_cycles(int device, unsigned* out, int capacity);
 
 // nvfp4_quant.cu
 void check_quant_shape(int rows, int K);
-void quantise(const void* x, int dtype, uint8_t* packed, uint8_t* scales, int rows, int K, cudaStream_t stream);
+// early: the kernel behind it may start while it runs (and waits for it on the device). Only for a caller that launches that
+// kernel itself and has it hold back its own dependents (GemmArgs::late_trigger). Otherwise a product two launches behind
+// the quantiser, told that the kernel in front of it leaves its operands alone, could read them before they are written.
+void quantise(const void* x, int dtype, uint8_t* packed, uint8_t* scales, int rows, int K, cudaStream_t stream, bool early = false);
 void quantise_scaled(const void* x, int dtype, float inv_global, uint8_t* packed, uint8_t* scales, int rows, int K,
                      cudaStream_t stream);
 void quantise_mx(const void* x, int dtype, uint8_t* packed, uint8_t* scales, int rows, int K, cudaStream_t stream);

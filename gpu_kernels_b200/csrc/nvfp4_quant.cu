@@ -10,6 +10,7 @@
 // written per value; a CTA owns a 128-row x 256-column tile so that each scale
 // atom (512 B) and each packed row segment (128 B) leaves in full lines.
 #include "nvfp4_internal.h"
+#include "ptx.cuh"
 #include "quant_device.cuh"
 
 #include <cuda_bf16.h>
@@ -23,14 +24,6 @@ namespace {
 constexpr int Q_ROWS = 128;      // rows per CTA tile = rows of one scale atom
 constexpr int Q_THREADS = 256;
 constexpr int MAX_GRID_Y = 32768;  // row tiles per layer of the grid
-
-// Launched through launch_chained(): the launch itself overlaps the tail of the kernel in front. A kernel behind this
-// one may set itself up only once the grid in front of THIS one has finished (the wait comes first): a product chained
-// behind a quantiser requests its weights before its own wait, and an earlier kernel may have written them.
-__device__ __forceinline__ void chain_point() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
 
 template <typename T> struct PairFormat { using type = void; };
 template <> struct PairFormat<__nv_bfloat16> { using type = Bf16Pairs; };
@@ -79,8 +72,11 @@ __device__ __forceinline__ uint32_t quantise_raw(const uint4 (&raw)[sizeof(T)], 
 template <typename T, int COLS, bool TAIL, bool SCALED>
 __global__ void __launch_bounds__(Q_THREADS, 4)
 quantise_kernel(const T* __restrict__ x, uint8_t* __restrict__ packed, uint8_t* __restrict__ scales,
-                int rows, int K, float inv_global) {
-    chain_point();
+                int rows, int K, float inv_global, int early) {
+    // Launched through launch_chained(): the launch itself overlaps the tail of the kernel in front. The wait comes first:
+    // a product behind this kernel requests its weights before its own wait, and an earlier kernel may have written them.
+    ptx::grid_dependency_wait();
+    if (early) ptx::grid_launch_dependents();
     constexpr int BLOCKS = COLS / 16;                           // 16-value blocks across the tile
     constexpr int ROWS_PER_PASS = Q_THREADS / BLOCKS;
     constexpr int PASSES = Q_ROWS / ROWS_PER_PASS;
@@ -179,7 +175,7 @@ dequantise_kernel(const uint8_t* __restrict__ packed, const uint8_t* __restrict_
 template <typename T>
 __global__ void __launch_bounds__(Q_THREADS, sizeof(T) == 2 ? 4 : 3)
 quantise_mx_kernel(const T* __restrict__ x, uint8_t* __restrict__ packed, uint8_t* __restrict__ scales, int rows, int K) {
-    chain_point();
+    ptx::grid_dependency_wait();
     constexpr int WORDS = 2 * int(sizeof(T));                  // 16-byte words of a block
     __shared__ __align__(16) uint8_t sf_tile[512];
     const int kb = threadIdx.x & 3, row_in_pass = threadIdx.x >> 2, row_base = int(blockIdx.x / unsigned(K / 128)) * Q_ROWS;
@@ -275,7 +271,7 @@ namespace {
 
 template <bool SCALED>
 void launch_quantise(const void* x, int dtype, float inv_global, uint8_t* packed, uint8_t* scales, int rows, int K,
-                     cudaStream_t stream) {
+                     bool early, cudaStream_t stream) {
     // 256-column tiles; 128-column ones when the grid would otherwise be less than two waves of resident CTAs
     // (four per SM). Measured, 128 / 256 columns: 4096 x 4096 bf16 12.3 / 14.4 us, 8192 x 8192 36.9 / 34.0 us.
     int device = 0, sms = 0;
@@ -289,7 +285,7 @@ void launch_quantise(const void* x, int dtype, float inv_global, uint8_t* packed
         const int row_tiles = (rows + Q_ROWS - 1) / Q_ROWS;
         const dim3 grid((K + cols - 1) / cols, std::min(row_tiles, MAX_GRID_Y), (row_tiles + MAX_GRID_Y - 1) / MAX_GRID_Y);
         auto go = [&](auto kernel) {
-            launch_chained(kernel, grid, dim3(Q_THREADS), size_t(0), stream, static_cast<const T*>(x), packed, scales, rows, K, inv_global);
+            launch_chained(kernel, grid, dim3(Q_THREADS), size_t(0), stream, static_cast<const T*>(x), packed, scales, rows, K, inv_global, early ? 1 : 0);
         };
         const bool tail = rows % Q_ROWS != 0;
         if (narrow) tail ? go(quantise_kernel<T, 128, true, SCALED>) : go(quantise_kernel<T, 128, false, SCALED>);
@@ -313,10 +309,10 @@ void check_quant_pointers(const void* x, const uint8_t* packed, const uint8_t* s
 
 }  // namespace
 
-void quantise(const void* x, int dtype, uint8_t* packed, uint8_t* scales, int rows, int K, cudaStream_t stream) {
+void quantise(const void* x, int dtype, uint8_t* packed, uint8_t* scales, int rows, int K, cudaStream_t stream, bool early) {
     check_quant_shape(rows, K);
     check_quant_pointers(x, packed, scales);
-    launch_quantise<false>(x, dtype, 1.0f, packed, scales, rows, K, stream);
+    launch_quantise<false>(x, dtype, 1.0f, packed, scales, rows, K, early, stream);
 }
 
 void quantise_scaled(const void* x, int dtype, float inv_global, uint8_t* packed, uint8_t* scales, int rows, int K,
@@ -324,7 +320,7 @@ void quantise_scaled(const void* x, int dtype, float inv_global, uint8_t* packed
     check_quant_shape(rows, K);
     check_quant_pointers(x, packed, scales);
     if (!(inv_global > 0.0f) || !(inv_global < 3.0e38f)) throw std::invalid_argument("nvfp4 quantise: the tensor scale must be positive and finite");
-    launch_quantise<true>(x, dtype, inv_global, packed, scales, rows, K, stream);
+    launch_quantise<true>(x, dtype, inv_global, packed, scales, rows, K, false, stream);
 }
 
 void check_mx_shape(int rows, int K) {

@@ -259,6 +259,53 @@ def test_overlapping_launches_with_static_operands(g, mode):
         plan.close()
 
 
+@pytest.mark.parametrize("quantiser", ["nvfp4", "scaled", "mx", "linear"])
+def test_static_operands_that_a_quantiser_two_launches_back_wrote(g, quantiser):
+    # the promise of "static_operands" is about the kernel in front: here a small product behind the quantiser that writes
+    # the operands (which takes longer than a launch, while the product in front leaves SMs free); "linear": quantiser and
+    # product in front are one call, and both plans are on the same A
+    from gpu_kernels_b200 import _lib
+    lib, mx = _lib.load(), quantiser == "mx"
+    m, n, k, per = 4096, 256, 8192, 32 if mx else 16
+    pb, sb = (g.quantize_mx if mx else g.quantize)(random_operand(n, k, seed=2, scale=0.02))
+    pa = torch.zeros((m, k // 2), dtype=torch.uint8, device="cuda")
+    sa = torch.zeros(m * k // per, dtype=torch.uint8, device="cuda")
+    front = g.Nvfp4Gemm(pa, pb, sa, sb) if quantiser == "linear" else g.Nvfp4Gemm(pb, pb, sb, sb, mx=mx)
+    plan = g.Nvfp4Gemm(pa, pb, sa, sb, mx=mx)
+    front_out = nan_output(front.m, front.n)
+
+    def quantise_and_front(x):
+        if quantiser == "linear":
+            front.linear(x, front_out)
+            return
+        args = (x.data_ptr(), 0, pa.data_ptr(), sa.data_ptr(), m, k, _lib.stream())
+        if quantiser == "scaled":
+            _lib.check(lib.gpu_kernels_nvfp4_quantize_scaled(*args[:2], 0.5, *args[2:]))
+        else:
+            _lib.check((lib.gpu_kernels_nvfp4_quantize_mx if mx else lib.gpu_kernels_nvfp4_quantize)(*args))
+        front.run(front_out)
+
+    xs = [random_operand(m, k, seed=60 + i) for i in range(4)]
+    wants = []
+    for x in xs:
+        quantise_and_front(x)
+        torch.cuda.synchronize()
+        wants.append(plan.run().clone())
+    for mode in (1, 2):
+        plan.set_option("static_operands", mode)
+        outs = [nan_output(m, n) for _ in xs]
+        for _ in range(5):
+            for x, out in zip(xs, outs):
+                quantise_and_front(x)
+                plan.run(out)
+        torch.cuda.synchronize()
+        assert all(torch.equal(out, want) for out, want in zip(outs, wants)), mode
+    plan.validate()
+    front.validate()
+    plan.close()
+    front.close()
+
+
 def test_distinct_scale_everywhere(g):
     # every (row, K block) has its own scale byte and codes are random nibbles: a wrong
     # scale column, swizzle or K-slice order cannot cancel out

@@ -1,0 +1,57 @@
+"""Who may let the next kernel start early (programmatic dependent launch), checked on the sources: the races this rules out
+need particular timing to show on a device.
+
+A kernel may read before its own wait what the kernel in front of it does not write (a product's weights, a routing plan,
+operands the caller declared static). What it reads must then be complete when the kernel in front lets it start: so a
+quantiser has no trigger unless the product directly behind it holds back its own dependents until it has finished."""
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parents[1] / "gpu_kernels_b200" / "csrc"
+WAIT = r"(?:ptx::)?grid_dependency_wait\(\);"
+TRIGGER = r"(?:ptx::)?grid_launch_dependents\(\);"
+
+
+def code(name):
+    lines = (re.sub(r"//.*", "", line).strip() for line in (CSRC / name).read_text().splitlines())
+    return "\n".join(line for line in lines if line)
+
+
+def first_statements(text, kernel):
+    body = re.search(r"\b" + kernel + r"\s*\([^{;]*\)\s*\{\n((?:.*\n){2})", text)
+    assert body, kernel
+    return body.group(1)
+
+
+def chained_kernels(text):
+    """Kernels that reach launch_chained() by name or through a local lambda that is given the kernel."""
+    return (set(re.findall(r"launch_chained\((\w+?)(?:<[^>]*>)?,", text)) - {"kernel"}) | set(re.findall(r"\bgo\((\w+)<", text))
+
+
+@pytest.mark.parametrize("kernel,trigger", [("quantise_kernel", "if (early) ptx::grid_launch_dependents();"), ("quantise_mx_kernel", None)])
+def test_quantisers_let_nothing_start_early_by_themselves(kernel, trigger):
+    text = code("nvfp4_quant.cu")
+    assert kernel in chained_kernels(text)
+    first, second = first_statements(text, kernel).splitlines()
+    assert re.fullmatch(WAIT, first)
+    assert second == trigger if trigger else "dependents" not in second
+    assert re.findall(r".*" + TRIGGER, text) == ["if (early) ptx::grid_launch_dependents();"]
+    # early: only for the linear call, whose product is launched with late_trigger
+    assert "launch_quantise<true>(x, dtype, inv_global, packed, scales, rows, K, false, stream);" in text
+    capi = code("nvfp4_capi.cu")
+    calls = re.findall(r"nvfp4_b200::quantise\(x(?:[^;]*\n?)*?;", capi)
+    early = [c for c in calls if re.search(r"true\s*\)\s*;$", c)]
+    assert len(calls) == 2 and len(early) == 1
+    behind = capi[capi.index(early[0]):]
+    assert behind.index("q.late_trigger = 1;") < behind.index("p.impl.launch(q,")
+
+
+def test_a_product_that_starts_late_waits_first():
+    text = code("nvfp4_gemm.cu")
+    triggers = re.findall(r".*\n.*" + TRIGGER, text)
+    late = [t for t in triggers if "if (g.late_trigger && threadIdx.x == 0)" in t]
+    assert len(triggers) == 3 and len(late) == 2
+    assert all(re.match(r".*" + WAIT, t) for t in late)
+    assert "g.late_trigger = p.late_trigger;" in text and "g.static_operands = g.late_trigger =" in text
