@@ -281,12 +281,12 @@ int gpu_kernels_nvfp4_linear(void* plan, const void* x, int dtype, void* C, void
         // front of the quantiser has finished, and the GEMM is told that the kernel in front of it leaves B alone, so
         // under programmatic dependent launch it sets itself up and requests its first tiles of B while the quantiser
         // runs, and waits for the quantiser's bytes only before its first load of A. Its own dependents start after
-        // that wait: another plan on the same A may be declared static.
+        // that wait (once its loads are requested): another plan on the same A may be declared static.
         nvfp4_b200::quantise(x, dtype, static_cast<uint8_t*>(const_cast<void*>(p.a)),
                              static_cast<uint8_t*>(const_cast<void*>(p.sfa)), p.params.M, p.params.K, s, true);
         gpu_kernels::Nvfp4Params q = p.params;
         if (q.static_operands != 1) q.static_operands = 1;      // 2 would let the GEMM read A before it is written
-        q.late_trigger = 1;
+        q.late_trigger = 2;
         p.impl.launch(q, static_cast<__half*>(C), s);
         nvfp4_b200::g_launches.fetch_add(1, std::memory_order_relaxed);
     });

@@ -225,10 +225,12 @@ struct GemmArgs {
     // stages of B are requested before the wait; 2 = none of the operands: only the epilogue waits, before its
     // first store, so the tiles of this launch run while the tail of the previous one drains.
     int static_operands;
-    // 1: the kernel behind this one may start only once the grid in front of this one has finished (the trigger comes
-    // after the wait instead of before it), as the kernel in front may itself have let this one start early: what it
-    // writes is then complete for any kernel behind this one, also for one that reads before its own wait.
-    // 0: at the start, which has the next launch set up sooner (256 cubed in a row: 3.92 us, 4.20 with 1).
+    // When the kernel behind this one may start. 0: at this one's start, which has it set up soonest (256 cubed in a row:
+    // 3.92 us, 4.20 with 1). 1, 2: only once the grid in front of this one has finished, as that one may itself have let
+    // this one start early: what it writes is then complete for any kernel behind this one, also for one that reads
+    // before its own wait. 1: right after the wait. 2 (with static_operands = 1): when this CTA has requested its last
+    // ring stage; until then the CTAs of the next kernel only get in the way of the loads (linear 8 x 8192 x 8192
+    // 13.86 us with 1, 13.28 with 2; 1000 x 8192 x 8192 38.0 and 37.2).
     int late_trigger;
     // EPI_DIRECT_RAGGED (one tile row, M = 128): the N columns are dealt to exactly as many tiles as there are
     // SMs, in units of 64 columns: the first ragged_extra tiles are ragged_base + 1 units wide, the others
@@ -472,6 +474,7 @@ struct Roles {
             }
         }
         if (early_b && issued < Cfg::STAGES) release_held(tmA, tmSFA, held, issued, who);   // fewer steps than ring stages
+        if (early_b && g.late_trigger == 2 && who == 0 && elect_one()) grid_launch_dependents();        // (release_held waited)
         if (PROF && lane == 0) {
             unsigned long long* out = g.prof + (size_t(unit) * CG + rank) * PROF_WORDS;
             out[PROF_PROD_WAIT] = waited;
@@ -769,7 +772,7 @@ struct Roles {
         // with static operands the prologue did not wait for the grid in front: nothing may be stored before it has finished
         if (g.static_operands != 0) {
             grid_dependency_wait();
-            if (g.late_trigger && threadIdx.x == 0) grid_launch_dependents();
+            if (g.late_trigger == 1 && threadIdx.x == 0) grid_launch_dependents();
         }
         Walk walk(g, unit, units, tiles, g.ksteps);
         Segment seg;

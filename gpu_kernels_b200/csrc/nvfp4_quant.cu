@@ -69,14 +69,15 @@ __device__ __forceinline__ uint32_t quantise_raw(const uint4 (&raw)[sizeof(T)], 
 // all row tiles: the last one as a launch of its own cost 1000 x 8192 bf16 another 4 us behind the 7 us of the others.
 // SCALED (two-level scaling): the values are first multiplied by the reciprocal of a per-tensor scale; the GEMM undoes
 // the tensor scales through its alpha.
-template <typename T, int COLS, bool TAIL, bool SCALED>
+// EARLY: the kernel behind this one may start while it runs (see quantise() in nvfp4_internal.h).
+template <typename T, int COLS, bool TAIL, bool SCALED, bool EARLY>
 __global__ void __launch_bounds__(Q_THREADS, 4)
 quantise_kernel(const T* __restrict__ x, uint8_t* __restrict__ packed, uint8_t* __restrict__ scales,
-                int rows, int K, float inv_global, int early) {
+                int rows, int K, float inv_global) {
     // Launched through launch_chained(): the launch itself overlaps the tail of the kernel in front. The wait comes first:
     // a product behind this kernel requests its weights before its own wait, and an earlier kernel may have written them.
     ptx::grid_dependency_wait();
-    if (early) ptx::grid_launch_dependents();
+    if constexpr (EARLY) ptx::grid_launch_dependents();
     constexpr int BLOCKS = COLS / 16;                           // 16-value blocks across the tile
     constexpr int ROWS_PER_PASS = Q_THREADS / BLOCKS;
     constexpr int PASSES = Q_ROWS / ROWS_PER_PASS;
@@ -269,9 +270,9 @@ void check_quant_shape(int rows, int K) {
 
 namespace {
 
-template <bool SCALED>
+template <bool SCALED, bool EARLY>
 void launch_quantise(const void* x, int dtype, float inv_global, uint8_t* packed, uint8_t* scales, int rows, int K,
-                     bool early, cudaStream_t stream) {
+                     cudaStream_t stream) {
     // 256-column tiles; 128-column ones when the grid would otherwise be less than two waves of resident CTAs
     // (four per SM). Measured, 128 / 256 columns: 4096 x 4096 bf16 12.3 / 14.4 us, 8192 x 8192 36.9 / 34.0 us.
     int device = 0, sms = 0;
@@ -285,11 +286,11 @@ void launch_quantise(const void* x, int dtype, float inv_global, uint8_t* packed
         const int row_tiles = (rows + Q_ROWS - 1) / Q_ROWS;
         const dim3 grid((K + cols - 1) / cols, std::min(row_tiles, MAX_GRID_Y), (row_tiles + MAX_GRID_Y - 1) / MAX_GRID_Y);
         auto go = [&](auto kernel) {
-            launch_chained(kernel, grid, dim3(Q_THREADS), size_t(0), stream, static_cast<const T*>(x), packed, scales, rows, K, inv_global, early ? 1 : 0);
+            launch_chained(kernel, grid, dim3(Q_THREADS), size_t(0), stream, static_cast<const T*>(x), packed, scales, rows, K, inv_global);
         };
         const bool tail = rows % Q_ROWS != 0;
-        if (narrow) tail ? go(quantise_kernel<T, 128, true, SCALED>) : go(quantise_kernel<T, 128, false, SCALED>);
-        else tail ? go(quantise_kernel<T, 256, true, SCALED>) : go(quantise_kernel<T, 256, false, SCALED>);
+        if (narrow) tail ? go(quantise_kernel<T, 128, true, SCALED, EARLY>) : go(quantise_kernel<T, 128, false, SCALED, EARLY>);
+        else tail ? go(quantise_kernel<T, 256, true, SCALED, EARLY>) : go(quantise_kernel<T, 256, false, SCALED, EARLY>);
     };
     switch (dtype) {
         case DTYPE_BF16: launch(__nv_bfloat16{}); break;
@@ -312,7 +313,8 @@ void check_quant_pointers(const void* x, const uint8_t* packed, const uint8_t* s
 void quantise(const void* x, int dtype, uint8_t* packed, uint8_t* scales, int rows, int K, cudaStream_t stream, bool early) {
     check_quant_shape(rows, K);
     check_quant_pointers(x, packed, scales);
-    launch_quantise<false>(x, dtype, 1.0f, packed, scales, rows, K, early, stream);
+    if (early) launch_quantise<false, true>(x, dtype, 1.0f, packed, scales, rows, K, stream);
+    else launch_quantise<false, false>(x, dtype, 1.0f, packed, scales, rows, K, stream);
 }
 
 void quantise_scaled(const void* x, int dtype, float inv_global, uint8_t* packed, uint8_t* scales, int rows, int K,
@@ -320,7 +322,7 @@ void quantise_scaled(const void* x, int dtype, float inv_global, uint8_t* packed
     check_quant_shape(rows, K);
     check_quant_pointers(x, packed, scales);
     if (!(inv_global > 0.0f) || !(inv_global < 3.0e38f)) throw std::invalid_argument("nvfp4 quantise: the tensor scale must be positive and finite");
-    launch_quantise<true>(x, dtype, inv_global, packed, scales, rows, K, false, stream);
+    launch_quantise<true, false>(x, dtype, inv_global, packed, scales, rows, K, stream);
 }
 
 void check_mx_shape(int rows, int K) {

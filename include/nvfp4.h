@@ -59,8 +59,9 @@ struct Nvfp4Params {
     // write B or SFB (weights): their first tiles are fetched while it drains; 2 = it writes none of A, B, SFA,
     // SFB: this launch computes while it drains and only holds back its stores of C until it has finished.
     int static_operands;
-    // 1: the kernel behind a launch may start only once the kernel in front of it has finished. For a launch behind a
-    // kernel that lets it start early and writes operands of other plans too (gpu_kernels_nvfp4_linear's quantiser).
+    // 1, 2: the kernel behind a launch may start only once the kernel in front of it has finished (2: and this launch has
+    // requested its last tiles). For a launch behind a kernel that lets it start early and writes operands of other plans
+    // too (gpu_kernels_nvfp4_linear's quantiser).
     int late_trigger;
     // Ragged tiling of a one-tile-row plan (M = 128) whose 256-column tiles would leave SMs without a tile:
     // ragged_units tiles (0 = off), the first ragged_extra of them ragged_base + 1 units of 64 columns wide, the

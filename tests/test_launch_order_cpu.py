@@ -30,28 +30,33 @@ def chained_kernels(text):
     return (set(re.findall(r"launch_chained\((\w+?)(?:<[^>]*>)?,", text)) - {"kernel"}) | set(re.findall(r"\bgo\((\w+)<", text))
 
 
-@pytest.mark.parametrize("kernel,trigger", [("quantise_kernel", "if (early) ptx::grid_launch_dependents();"), ("quantise_mx_kernel", None)])
+@pytest.mark.parametrize("kernel,trigger", [("quantise_kernel", "if constexpr (EARLY) ptx::grid_launch_dependents();"), ("quantise_mx_kernel", None)])
 def test_quantisers_let_nothing_start_early_by_themselves(kernel, trigger):
     text = code("nvfp4_quant.cu")
     assert kernel in chained_kernels(text)
     first, second = first_statements(text, kernel).splitlines()
     assert re.fullmatch(WAIT, first)
     assert second == trigger if trigger else "dependents" not in second
-    assert re.findall(r".*" + TRIGGER, text) == ["if (early) ptx::grid_launch_dependents();"]
+    assert re.findall(r".*" + TRIGGER, text) == ["if constexpr (EARLY) ptx::grid_launch_dependents();"]
     # early: only for the linear call, whose product is launched with late_trigger
-    assert "launch_quantise<true>(x, dtype, inv_global, packed, scales, rows, K, false, stream);" in text
+    assert re.findall(r"(.*)launch_quantise<\w+, true>\(", text) == ["if (early) "]
     capi = code("nvfp4_capi.cu")
     calls = re.findall(r"nvfp4_b200::quantise\(x(?:[^;]*\n?)*?;", capi)
     early = [c for c in calls if re.search(r"true\s*\)\s*;$", c)]
     assert len(calls) == 2 and len(early) == 1
     behind = capi[capi.index(early[0]):]
-    assert behind.index("q.late_trigger = 1;") < behind.index("p.impl.launch(q,")
+    assert behind.index("q.late_trigger = 2;") < behind.index("p.impl.launch(q,")
 
 
-def test_a_product_that_starts_late_waits_first():
+def test_a_product_that_triggers_late_waits_first():
     text = code("nvfp4_gemm.cu")
     triggers = re.findall(r".*\n.*" + TRIGGER, text)
-    late = [t for t in triggers if "if (g.late_trigger && threadIdx.x == 0)" in t]
-    assert len(triggers) == 3 and len(late) == 2
-    assert all(re.match(r".*" + WAIT, t) for t in late)
+    assert len(triggers) == 4
+    assert sum("if (threadIdx.x == 0 && !g.late_trigger)" in t for t in triggers) == 1
+    after_wait = [t for t in triggers if re.search(r"if \(g\.late_trigger(?: == 1)? && threadIdx\.x == 0\)", t)]
+    assert len(after_wait) == 2 and all(re.match(r".*" + WAIT, t) for t in after_wait)
+    # the producer's: behind its last load, and release_held waits before its first load of A
+    last = [t for t in triggers if "g.late_trigger == 2" in t]
+    assert len(last) == 1 and last[0].startswith("if (early_b && issued < Cfg::STAGES) release_held(") and "\nif (early_b && " in last[0]
+    assert re.search(r"void release_held\([^{]*\{\n" + WAIT, text)
     assert "g.late_trigger = p.late_trigger;" in text and "g.static_operands = g.late_trigger =" in text
