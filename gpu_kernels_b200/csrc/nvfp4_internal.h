@@ -75,8 +75,9 @@ struct GroupedGemm {
     const int* num_blocks;
     const int* block_valid;     // real rows per block (device, from the plan kernel); null = every row of C is written
     // 1: B, its scales, block_expert and num_blocks are complete once the grid IN FRONT OF the kernel in front of a
-    // launch has finished, and that kernel triggers its dependents only after its own wait: the launch reads them before
-    // its own wait, so its first weight tiles are on their way while that kernel runs.
+    // launch has finished, and that kernel triggers its dependents only after its own wait (every kernel of the expert
+    // path does): the launch reads them before its own wait, so its first weight tiles are on their way while that kernel
+    // runs.
     int static_weights;
 };
 void grouped_prepare(GroupedGemm& p, const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB,

@@ -35,17 +35,11 @@ constexpr int PAYLOAD_TAIL = 16;          // route weight (float) + padding, kee
 
 __host__ __device__ inline int payload_bytes(int hidden) { return hidden / 2 + hidden / 16 + PAYLOAD_TAIL; }
 
-// Every kernel of this file opens with chain_point(): it lets the kernel behind it in the stream be scheduled
-// early and then waits until the kernel in front of it has finished, so under programmatic dependent launch
-// the launch latencies of the forward's dozen small kernels overlap instead of adding up. Launched through
-// launch_chained() (the attribute that permits the early start); an ordinary launch behaves as before.
-__device__ __forceinline__ void chain_point() {
-    ptx::grid_launch_dependents();
-    ptx::grid_dependency_wait();
-}
-
+// Every kernel of this file but the barrier opens with ptx::chain_point() and is launched through launch_chained() (the
+// attribute that permits the early start): under programmatic dependent launch the launch latencies of the forward's
+// dozen small kernels overlap instead of adding up. An ordinary launch behaves as before.
 __global__ void route_count_kernel(const long long* __restrict__ ids, int routes, int experts, int* __restrict__ counts) {
-    chain_point();
+    ptx::chain_point();
     extern __shared__ int local[];
     for (int e = threadIdx.x; e < experts; e += blockDim.x) local[e] = 0;
     __syncthreads();
@@ -98,7 +92,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(int* __restrict__ bl
                             int* __restrict__ seg_pool_offset, int* __restrict__ block_expert,
                             int* __restrict__ num_blocks, int* __restrict__ totals, int* __restrict__ peer_offset,
                             const long long* __restrict__ ids, int routes, int* __restrict__ cursor, int peer_to_pool) {
-    chain_point();
+    ptx::chain_point();
     extern __shared__ int sh[];
     const int local_experts = experts / world;
     const int segments = world * local_experts;          // == experts
@@ -208,7 +202,7 @@ __global__ void pack_kernel(const uint8_t* __restrict__ xq, const uint8_t* __res
                             uint8_t* __restrict__ send_rows, int* __restrict__ send_pos,
                             const int* __restrict__ seg_pool_offset, uint8_t* __restrict__ pool_packed,
                             uint8_t* __restrict__ pool_scales, float* __restrict__ pool_weight) {
-    chain_point();
+    ptx::chain_point();
     const int lane = threadIdx.x & 31;
     const int route = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (route >= routes) return;
@@ -248,7 +242,7 @@ __global__ void unpack_kernel(const uint8_t* __restrict__ recv_rows, const int* 
                               uint8_t* __restrict__ pool_packed, uint8_t* __restrict__ pool_scales,
                               float* __restrict__ pool_weight, int* __restrict__ pool_of_recv, int local_experts,
                               int* __restrict__ pool_dst) {
-    chain_point();
+    ptx::chain_point();
     const int lane = threadIdx.x & 31;
     const int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (p >= totals[0] || totals[2]) return;
@@ -285,7 +279,7 @@ __global__ void unpack_meta_kernel(const uint8_t* __restrict__ side, const int* 
                                    const int* __restrict__ seg_src_offset, const int* __restrict__ seg_pool_offset,
                                    uint8_t* __restrict__ pool_scales, float* __restrict__ pool_weight,
                                    int* __restrict__ pool_dst, int local_experts) {
-    chain_point();
+    ptx::chain_point();
     const int lane = threadIdx.x & 31;
     const int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (p >= totals[0] || totals[2]) return;
@@ -313,7 +307,7 @@ __global__ void __launch_bounds__(256)
 swiglu_quant_kernel(const __nv_bfloat16* __restrict__ gate_up, const float* __restrict__ pool_weight,
                     const int* __restrict__ num_blocks, int block_rows, int inter, float clamp,
                     uint8_t* __restrict__ act_packed, uint8_t* __restrict__ act_scales) {
-    chain_point();
+    ptx::chain_point();
     __shared__ __align__(16) uint8_t sf_tile[4 * 512];
     if (int(blockIdx.y) * 128 >= *num_blocks * block_rows) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -368,7 +362,7 @@ swiglu_quant_kernel(const __nv_bfloat16* __restrict__ gate_up, const float* __re
 
 __global__ void return_rows_kernel(const uint4* __restrict__ out_pool, const int* __restrict__ pool_of_recv,
                                    const int* __restrict__ totals, int row_vec, uint4* __restrict__ ret) {
-    chain_point();
+    ptx::chain_point();
     const int p = blockIdx.x;
     if (p >= totals[0] || totals[2]) return;
     const uint4* src = out_pool + size_t(pool_of_recv[p]) * row_vec;
@@ -385,7 +379,7 @@ template <int TOPK>
 __global__ void __launch_bounds__(256)
 reduce_kernel(const uint4* __restrict__ returned, const int* __restrict__ send_pos, int topk,
               int row_vec, uint4* __restrict__ y, const long long* __restrict__ ids, int experts) {
-    chain_point();
+    ptx::chain_point();
     const int t = blockIdx.x;
     constexpr int SLOTS = TOPK > 0 ? TOPK : 1;
     const int count = TOPK > 0 ? TOPK : topk;
@@ -448,7 +442,7 @@ __global__ void pack_peer_kernel(const uint8_t* __restrict__ xq, const uint8_t* 
                                  const long long* __restrict__ ids, const float* __restrict__ weights, int routes,
                                  int topk, int hidden, int local_experts, int experts, const int* __restrict__ peer_offset,
                                  int* __restrict__ cursor, PeerBuffers recv, int recv_capacity, int* __restrict__ error) {
-    chain_point();
+    ptx::chain_point();
     const int lane = threadIdx.x & 31;
     const int route = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (route >= routes) return;
@@ -492,9 +486,7 @@ quantise_route_kernel(const __nv_bfloat16* __restrict__ x, const long long* __re
                       int* __restrict__ error,
                       uint8_t* __restrict__ pool_packed, uint8_t* __restrict__ pool_scales,
                       float* __restrict__ pool_weight, int* __restrict__ route_row) {
-    // the wait before the trigger: the first expert GEMM behind this kernel reads the routing plan before its own wait
-    ptx::grid_dependency_wait();
-    ptx::grid_launch_dependents();
+    ptx::chain_point();
     extern __shared__ __align__(16) uint8_t smem_rows[];        // ROUTE_BUFFERS x (codes [hidden/2] | scale bytes [hidden/16] | int dst[topk])
     const int row_bytes = hidden / 2 + hidden / 16;
     const int dst_off = (row_bytes + 15) & ~15;
@@ -627,7 +619,7 @@ __global__ void return_peer_kernel(const uint4* __restrict__ out_pool, const uin
                                    const int* __restrict__ pool_of_recv, const int* __restrict__ totals,
                                    const int* __restrict__ seg_src_offset, int segments, int local_experts, int hidden,
                                    PeerBuffers slots, int slot_capacity, int* __restrict__ error) {
-    chain_point();
+    ptx::chain_point();
     const int p = blockIdx.x;
     if (p >= totals[0] || totals[2]) return;
     int lo = 0, hi = segments;
@@ -819,7 +811,7 @@ void moe_quantise_route(const void* x_bf16, const long long* ids, const float* w
 __global__ void __launch_bounds__(256)
 clear_live_kernel(const int* __restrict__ num_blocks, int block_rows, int hidden, uint8_t* __restrict__ pool_scales,
                   float* __restrict__ pool_weight, int* __restrict__ pool_dst) {
-    chain_point();
+    ptx::chain_point();
     const int row0 = blockIdx.x * 128;
     if (row0 >= *num_blocks * block_rows) return;
     const size_t bytes = size_t(hidden / 64) * 512;            // the scale atoms of 128 rows

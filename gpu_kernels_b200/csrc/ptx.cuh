@@ -63,6 +63,13 @@ __device__ __forceinline__ void grid_launch_dependents() {
 __device__ __forceinline__ void grid_dependency_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+// Wait, then let the next kernel start. A kernel that opens with it may rely, before its own wait, on everything older
+// than the kernel in front of it if that one opens with it too: with the trigger first it could start while the last CTAs
+// of a kernel two launches back are still writing.
+__device__ __forceinline__ void chain_point() {
+    grid_dependency_wait();
+    grid_launch_dependents();
+}
 
 // ---- mbarrier -------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t arrivals) {

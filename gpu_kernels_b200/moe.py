@@ -153,8 +153,9 @@ class Nvfp4MoE:
                 _lib.check(lib.gpu_kernels_nvfp4_grouped_set_valid_rows(fc1, self.block_valid.data_ptr()))
                 _lib.check(lib.gpu_kernels_nvfp4_grouped_set_valid_rows(fc2, self.block_valid.data_ptr()))
                 if self.world == 1 and fused and fused_dispatch:
-                    # The routing plan is two kernels back for FC1 (behind the dispatch) and three for FC2, and both
-                    # kernels in front trigger after their wait: each GEMM requests its first weights while they run.
+                    # The routing plan is at least two kernels back for FC1 (behind the dispatch, or the pack kernel
+                    # where fused_dispatch was switched off since) and three for FC2, and every kernel of the path
+                    # triggers after its wait: each GEMM requests its first weights while the kernel in front runs.
                     _lib.check(lib.gpu_kernels_nvfp4_grouped_set_static_weights(fc1, 1))
                     _lib.check(lib.gpu_kernels_nvfp4_grouped_set_static_weights(fc2, 1))
                 self._plans[rows] = (fc1, fc2)

@@ -188,7 +188,7 @@ void gpu_kernels_nvfp4_grouped_plan_destroy(void* plan);
 int gpu_kernels_nvfp4_grouped_set_valid_rows(void* plan, const void* block_valid);
 /* on = 1: the caller promises that B, its scales, block_expert and num_blocks are complete once the grid in front of the
  * kernel in front of each launch has finished, and that this kernel triggers its dependents only after its own wait (the
- * dispatch kernel does, and a grouped launch with this option does). The launch then requests its first weight tiles
+ * routing, dispatch, pack and activation kernels do, and a grouped launch with this option does). The launch then requests its first weight tiles
  * while that kernel runs. 0 (default): nothing is read before the wait. Ignored by gpu_kernels_nvfp4_grouped_run_scatter. */
 int gpu_kernels_nvfp4_grouped_set_static_weights(void* plan, int on);
 int gpu_kernels_nvfp4_grouped_run(void* plan, void* C, int out_bf16, void* stream);

@@ -2,8 +2,9 @@
 need particular timing to show on a device.
 
 A kernel may read before its own wait what the kernel in front of it does not write (a product's weights, a routing plan,
-operands the caller declared static). What it reads must then be complete when the kernel in front lets it start: so a
-quantiser has no trigger unless the product directly behind it holds back its own dependents until it has finished."""
+operands the caller declared static). What it reads must then be complete when the kernel in front lets it start: so the
+expert path's kernels wait before their trigger, and a quantiser has no trigger unless the product directly behind it
+holds back its own dependents until the quantiser has finished."""
 import re
 from pathlib import Path
 
@@ -28,6 +29,22 @@ def first_statements(text, kernel):
 def chained_kernels(text):
     """Kernels that reach launch_chained() by name or through a local lambda that is given the kernel."""
     return (set(re.findall(r"launch_chained\((\w+?)(?:<[^>]*>)?,", text)) - {"kernel"}) | set(re.findall(r"\bgo\((\w+)<", text))
+
+
+def test_chain_point_waits_first():
+    assert re.search(r"void chain_point\(\) \{\n" + WAIT + "\n" + TRIGGER + r"\n\}", code("ptx.cuh"))
+    for path in CSRC.iterdir():
+        if path.suffix in (".cu", ".cuh", ".h") and path.name != "ptx.cuh":
+            assert "griddepcontrol" not in code(path.name), f"{path.name}: raw instruction"
+
+
+def test_expert_path_kernels_wait_first():
+    text = code("nvfp4_moe.cu")
+    kernels = chained_kernels(text)
+    assert {"plan_kernel", "pack_kernel", "swiglu_quant_kernel", "quantise_route_kernel", "reduce_kernel"} <= kernels
+    for kernel in kernels:
+        assert first_statements(text, kernel).startswith("ptx::chain_point();"), kernel
+    assert not re.search(TRIGGER, text)
 
 
 @pytest.mark.parametrize("kernel,trigger", [("quantise_kernel", "if constexpr (EARLY) ptx::grid_launch_dependents();"), ("quantise_mx_kernel", None)])

@@ -199,6 +199,26 @@ def test_fused_dispatch_matches_quantise_then_pack(g):
         assert np.array_equal(pools[0][1][real], pools[1][1][real])
 
 
+def test_dispatch_changed_after_construction(g):
+    # a layer built for the fused dispatch and then switched to the stand-alone quantiser: the first product still reads
+    # the routing plan of its own batch (its blocks' experts change from call to call)
+    tokens, hidden, inter, experts, topk = 200, 512, 256, 16, 4
+    x, logits, w1, w2 = make_layer(9, tokens, hidden, inter, experts, topk, skew=True)
+    layer = g.Nvfp4MoE(w1, w2, experts, topk, max_tokens=256)
+    plain = g.Nvfp4MoE(w1, w2, experts, topk, max_tokens=256, fused_dispatch=False)
+    batches = [g.route(torch.roll(logits, 3 * i, dims=1), topk) for i in range(6)]
+    wants = [plain(x, ids, wts).clone() for ids, wts in batches]
+    torch.cuda.synchronize()
+    for fused_dispatch in (False, True, False):
+        layer.fused_dispatch = fused_dispatch
+        got = [layer(x, ids, wts).clone() for ids, wts in batches]
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(got, wants)), fused_dispatch
+    layer.check()
+    layer.close()
+    plain.close()
+
+
 @pytest.mark.parametrize("world,experts,block_rows", [(2, 8, 128), (4, 32, 256), (8, 256, 128)])
 def test_plan_agrees_across_ranks_on_pool_rows(g, world, experts, block_rows):
     # every rank derives, from the same gathered counts, where ITS rows start in the pool of each expert's
