@@ -39,6 +39,7 @@ SIGNATURES = {
     "gpu_kernels_nvfp4_peer_exchange": ([P, P, I, I, P, I, I, P, P], I),
     "gpu_kernels_nvfp4_plan_set_gather": ([P, ctypes.POINTER(P), I, I, I], I),
     "gpu_kernels_nvfp4_plan_info": ([P, ctypes.POINTER(I)], I),
+    "gpu_kernels_nvfp4_plan_launch_info": ([P, ctypes.POINTER(I)], I),
     "gpu_kernels_nvfp4_plan_placement_misses": ([P, ctypes.POINTER(ctypes.c_uint)], I),
     "gpu_kernels_nvfp4_side_route": ([ctypes.c_char_p, I, I, ctypes.POINTER(ctypes.c_uint)], I),
     "gpu_kernels_nvfp4_l2_census": ([ctypes.POINTER(ctypes.c_uint), I, ctypes.POINTER(I)], I),

@@ -19,6 +19,7 @@
 namespace nvfp4_b200 {
 extern std::atomic<unsigned long long> g_launches;
 int gemm_stage_count(int cta_group, int tile_n, int direct_store);
+void gemm_launch_info(const gpu_kernels::Nvfp4Params& p, int* info);
 void validate_device_slot(int device);
 unsigned last_kernel_cycles();
 int gemm_profile(const gpu_kernels::Nvfp4Params& p, __half* C, cudaStream_t stream, unsigned long long* host, int max_words);
@@ -366,6 +367,10 @@ int gpu_kernels_nvfp4_plan_set_option(void* plan, const char* key, int value) {
             const int tiles_m = p.params.M / (128 * p.params.cta_group);
             if (value < 1) throw std::invalid_argument("set_option: group_m must be >= 1");
             p.params.group_m = value < tiles_m ? value : tiles_m;
+            if (p.params.plain_tile_n) {                         // the band order of the tiles a plain launch takes
+                const int rows = 128 * p.params.plain_cta_group, plain_m = (p.params.M + rows - 1) / rows;
+                p.params.plain_group_m = value < plain_m ? value : plain_m;
+            }
         } else if (std::strcmp(key, "c_evict_first") == 0) {
             p.params.c_evict_first = value ? 1 : 0;
         } else if (std::strcmp(key, "direct_store") == 0) {
@@ -429,6 +434,14 @@ int gpu_kernels_nvfp4_plan_info(void* plan, int* info) {
                                 q.direct_store, q.out_bf16, q.route ? 1 : 0, q.side_units[0], q.side_units[1],
                                 q.ragged_units};
         std::memcpy(info, values, sizeof(values));
+    });
+}
+
+int gpu_kernels_nvfp4_plan_launch_info(void* plan, int* info) {
+    return guarded([&] {
+        Plan& p = as_plan(plan);
+        if (!info) throw std::invalid_argument("plan_launch_info: null output");
+        nvfp4_b200::gemm_launch_info(p.params, info);
     });
 }
 

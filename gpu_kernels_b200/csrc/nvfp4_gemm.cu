@@ -1268,7 +1268,7 @@ void choose_plain_tiles(gpu_kernels::Nvfp4Params& p, const uint8_t* B, int force
     p.plain_cta_group = best->cta_group;
     p.plain_tile_n = best->tile_n;
     p.plain_units = std::min(fit_units(p.device, best->cta_group, best->tile_n), tiles(*best));
-    p.plain_group_m = band_rows(p.plain_units, tiles_m);
+    p.plain_group_m = std::max(1, std::min(env_int("NVFP4_B200_GROUP_M", band_rows(p.plain_units, tiles_m)), tiles_m));
     p.plain_B = operand_map(B, p.N, p.K, best->tile_n / best->cta_group);
 }
 
@@ -1508,6 +1508,20 @@ void launch_dense(const gpu_kernels::Nvfp4Params& p, const CUtensorMap& tmC, con
     }
 }
 
+// Whether a launch takes the tiles of choose_plain_tiles.
+bool takes_plain_tiles(const gpu_kernels::Nvfp4Params& p) {
+    return p.plain_tile_n && p.split_k <= 1 && !p.gather_world && !p.ragged_units && !p.route && p.direct_store;
+}
+
+// Twins: one tile per CTA, and a K loop long enough to pay for the larger block and the second accumulator.
+// Measured (us, one issuer / two): 32 steps 8 x 8192 x 8192 12.8 / 11.5, 1 x 2048 x 8192 12.3 / 10.2; 28 steps
+// 384 x 1536 x 7168 11.4 / 9.6; 16 steps 64 x 4096 x 4096 8.0 / 7.6, 8 x 14336 x 4096 9.5 / 9.5; 8 steps
+// 300 x 2048 x 2048 5.7 / 6.0; 2 steps 1 x 4096 x 512 3.4 / 4.3.
+bool plain_twins(const gpu_kernels::Nvfp4Params& p) {
+    const int tiles = ((p.M + 127) / 128) * ((p.N + p.plain_tile_n - 1) / p.plain_tile_n);
+    return p.plain_cta_group == 1 && p.plain_tile_n <= 128 && tiles <= p.plain_units && (p.K + STAGE_K - 1) / STAGE_K >= 16;
+}
+
 // A plain launch on the tiles of choose_plain_tiles.
 template <int CG, int UN>
 void launch_plain(const gpu_kernels::Nvfp4Params& p, const CUtensorMap& tmC, const GemmArgs& dense, cudaStream_t stream) {
@@ -1517,11 +1531,7 @@ void launch_plain(const gpu_kernels::Nvfp4Params& p, const CUtensorMap& tmC, con
     g.group_m = p.plain_group_m;
     const bool pdl = p.pdl != 0;
     if constexpr (CG == 1 && UN <= 128) {
-        // Twins: one tile per CTA, and a K loop long enough to pay for the larger block and the second accumulator.
-        // Measured (us, one issuer / two): 32 steps 8 x 8192 x 8192 12.8 / 11.5, 1 x 2048 x 8192 12.3 / 10.2; 28 steps
-        // 384 x 1536 x 7168 11.4 / 9.6; 16 steps 64 x 4096 x 4096 8.0 / 7.6, 8 x 14336 x 4096 9.5 / 9.5; 8 steps
-        // 300 x 2048 x 2048 5.7 / 6.0; 2 steps 1 x 4096 x 512 3.4 / 4.3.
-        if (g.tiles_m * g.tiles_n <= p.plain_units && g.ksteps >= 16) {
+        if (plain_twins(p)) {
             if (p.mx) launch_instance<1, UN, EPI_DIRECT_TWIN, false, true>(p.device, p.plain_units, p.A, p.plain_B, p.SFA, p.SFB, tmC, g, stream, pdl);
             else launch_instance<1, UN, EPI_DIRECT_TWIN>(p.device, p.plain_units, p.A, p.plain_B, p.SFA, p.SFB, tmC, g, stream, pdl);
             return;
@@ -1539,7 +1549,7 @@ void launch_with(const gpu_kernels::Nvfp4Params& p, void* C, cudaStream_t stream
     // only the staged route stores C through a map
     const CUtensorMap tmC = p.direct_store ? CUtensorMap{} : output_map(C, p.M, p.N, p.out_bf16 != 0);
     const GemmArgs g = dense_args(p, C, prof);
-    if (p.plain_tile_n && p.split_k <= 1 && !p.gather_world && !p.ragged_units && !p.route && p.direct_store && !prof) {
+    if (takes_plain_tiles(p) && !prof) {
         if (p.plain_cta_group == 2) launch_plain<2, 256>(p, tmC, g, stream);
         else if (p.plain_tile_n == 256) launch_plain<1, 256>(p, tmC, g, stream);
         else if (p.plain_tile_n == 128) launch_plain<1, 128>(p, tmC, g, stream);
@@ -1603,6 +1613,16 @@ void require_sm100() {
 
 // Plain launch through a pointer that may be FP16 or BF16 storage (the plan's out_bf16 decides).
 void gemm_launch(const gpu_kernels::Nvfp4Params& p, void* C, cudaStream_t stream) { launch_with(p, C, stream, nullptr); }
+
+// What gemm_launch runs for this plan: {cta_group, tile_n, units, group_m, issuers}.
+void gemm_launch_info(const gpu_kernels::Nvfp4Params& p, int* info) {
+    const bool plain = takes_plain_tiles(p);
+    info[0] = plain ? p.plain_cta_group : p.cta_group;
+    info[1] = plain ? p.plain_tile_n : p.tile_n;
+    info[2] = plain ? p.plain_units : p.ragged_units ? p.ragged_units : p.clusters;
+    info[3] = plain ? p.plain_group_m : p.group_m;
+    info[4] = plain && plain_twins(p) ? 2 : 1;
+}
 
 // The device-wide slot (grouped launches and the expert-path kernels report there).
 void validate_device_slot(int device) { validate_slot(device, 0); }

@@ -62,11 +62,15 @@ class Nvfp4Gemm:
             self.out_dtype = torch.bfloat16 if value else torch.float16
 
     def info(self) -> dict:
-        buf = (ctypes.c_int * 16)()
+        """The plan's own tiles and options, and under launch_... what `run` launches as the options stand: a plain launch
+        takes other tiles than the plan's own where they finish the shape sooner."""
+        buf, launch = (ctypes.c_int * 16)(), (ctypes.c_int * 5)()
         _lib.check(_lib.load().gpu_kernels_nvfp4_plan_info(self._plan, buf))
         keys = ("M", "N", "K", "units", "cta_group", "tile_n", "group_m", "stages", "split_k", "k_skew",
                 "direct_store", "out_bf16", "l2_side", "side0_units", "side1_units", "ragged_tiles")
-        return dict(zip(keys, list(buf)))
+        _lib.check(_lib.load().gpu_kernels_nvfp4_plan_launch_info(self._plan, launch))
+        launch_keys = ("launch_cta_group", "launch_tile_n", "launch_units", "launch_group_m", "launch_issuers")
+        return dict(zip(keys + launch_keys, list(buf) + list(launch)))
 
     def placement_misses(self) -> int:
         """Clusters (summed over launches) that ran on the other L2 side than the tile route assumed."""
@@ -99,7 +103,7 @@ class Nvfp4Gemm:
         return out
 
     def profile(self, out: torch.Tensor):
-        """One launch with the kernel's per-role wait counters on. Returns a list of dicts, one per CTA."""
+        """One launch, on the plan's own tiles, with the kernel's per-role wait counters on. Returns a list of dicts, one per CTA."""
         n = 4096 * 16
         buf = (ctypes.c_ulonglong * n)()
         written = ctypes.c_int()

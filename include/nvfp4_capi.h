@@ -131,8 +131,13 @@ int gpu_kernels_nvfp4_plan_set_option(void* plan, const char* key, int value);
  * off. Not inside stream capture (synchronises once). */
 int gpu_kernels_nvfp4_plan_set_gather(void* plan, void* const* buffers, int world, int col0, int n_total);
 /* Fills info[0..15] = {M, N, K, units, cta_group, tile_n, group_m, stages, split_k, k_skew, direct_store,
- * out_bf16, l2_side order in use, clusters on L2 side 0, on side 1, ragged tiles (0 = uniform tiling)}. */
+ * out_bf16, l2_side order in use, clusters on L2 side 0, on side 1, ragged tiles (0 = uniform tiling)}: the plan's own
+ * tiles, whole tiles of the padded shape. */
 int gpu_kernels_nvfp4_plan_info(void* plan, int* info);
+/* Fills info[0..4] = {cta_group, tile_n, units, group_m, issuers} of what gpu_kernels_nvfp4_custom launches for this plan
+ * as its options stand: a plain launch takes other tiles than the plan's own where they finish the shape sooner. issuers
+ * = 2: even and odd K steps are summed apart and added at the end. */
+int gpu_kernels_nvfp4_plan_launch_info(void* plan, int* info);
 
 /* With the "l2_side" order: how many clusters, summed over this plan's launches, found themselves on the
  * other side of the L2 than the plan's tile route assumed (they lose locality, nothing else). Synchronising copy. */
@@ -146,7 +151,7 @@ int gpu_kernels_nvfp4_side_route(const unsigned char* unit_side, int units, int 
  * indexed by SM id (0 = no CTA ran there); *written = 0 when no census has run on this device yet. */
 int gpu_kernels_nvfp4_l2_census(unsigned* cycles_by_sm, int capacity, int* written);
 
-/* Diagnostic: one launch with per-role wait counters on; writes 16 words per CTA
+/* Diagnostic: one launch, on the plan's own tiles (plan_info), with per-role wait counters on; writes 16 words per CTA
  * {producer wait, producer total, MMA wait-for-data, MMA wait-for-accumulator, MMA total, epilogue
  * wait-for-accumulator, epilogue wait-for-store, epilogue total, SM id, ...} in SM clock cycles.
  * Allocates and frees a small device buffer and synchronises the stream. */

@@ -338,6 +338,30 @@ def test_alpha_and_group_m(g):
         assert torch.equal(again, base), f"tile order group_m={gm} changed the result"
 
 
+@pytest.mark.parametrize("m,n,k,tile", [(1024, 1536, 512, 1128), (1100, 4360, 1088, 2256), (4096, 4096, 512, 2256)])
+def test_group_m_reaches_the_tiles_that_are_launched(g, m, n, k, tile, monkeypatch):
+    # narrow tiles and CTA pairs where the plan's own tiles are others, and a plan that runs its own; by option and by
+    # environment, clamped to the tile rows: another order of the tiles, the same bits
+    pa, sa = g.quantize(random_operand(m, k, seed=13))
+    pb, sb = g.quantize(random_operand(n, k, seed=14))
+    plan = g.Nvfp4Gemm(pa, pb, sa, sb)
+    info = plan.info()
+    assert info["launch_cta_group"] * 1000 + info["launch_tile_n"] == tile, info
+    tile_rows = -(-m // (128 * info["launch_cta_group"]))
+    base = plan.run(nan_output(m, n)).clone()
+    for gm in (1, 2, 3, 100):
+        plan.set_option("group_m", gm)
+        assert plan.info()["launch_group_m"] == min(gm, tile_rows)
+        assert torch.equal(plan.run(nan_output(m, n)), base), f"tile order group_m={gm} changed the result"
+    plan.validate()
+    plan.close()
+    monkeypatch.setenv("NVFP4_B200_GROUP_M", "3")
+    plan = g.Nvfp4Gemm(pa, pb, sa, sb)
+    assert plan.info()["launch_group_m"] == min(3, tile_rows)
+    assert torch.equal(plan.run(nan_output(m, n)), base)
+    plan.close()
+
+
 def test_matches_cublaslt(g):
     m = n = k = 1024
     pa, sa = g.quantize(random_operand(m, k, seed=21))
