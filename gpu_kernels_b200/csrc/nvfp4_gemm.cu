@@ -238,7 +238,7 @@ struct GemmArgs {
     // fetched in 64-row boxes; a tile's scale atoms are the two 128-row blocks its columns lie in, and the MMA
     // reads them from the column (n0 % 128) / 32 on.
     int ragged_base, ragged_extra;
-    // Rows of A's box (CG = 1): 128, or M rounded up to 8 rows when M < 128. The rows of the stage a smaller box does
+    // Rows of A's box: 128, or M rounded up to 8 rows when M < 128. The rows of the stage a smaller box does
     // not reach keep whatever bytes they hold: every E2M1 code is finite, a row of the product depends on its own row
     // of A alone, and rows >= M are never stored.
     int a_box_rows;
@@ -384,10 +384,9 @@ struct Roles {
                     sfb_live = min(Cfg::SFB_BLOCKS, blocks - sfb_block);
                     const int first_b = tn * UN;
                     const int live_b = CG == 2 ? 1 + int(first_b + Cfg::B_ROWS < g.N) : 1;       // boxes of the pair
-                    stage_bytes = uint32_t(g.a_box_rows * ROW_BYTES + Cfg::SFA_BYTES + sfb_live * Cfg::SFB_BLOCK_BYTES) * CG +
-                                  uint32_t(live_b * Cfg::B_BYTES);
                     const int live_a = CG == 2 ? 1 + int(tm * Cfg::TILE_M + BLOCK_M < g.M) : 1;
-                    if (live_a < CG) stage_bytes -= uint32_t(Cfg::A_BYTES + Cfg::SFA_BYTES);
+                    stage_bytes = uint32_t(live_a * (g.a_box_rows * ROW_BYTES + Cfg::SFA_BYTES) + CG * sfb_live * Cfg::SFB_BLOCK_BYTES +
+                                           live_b * Cfg::B_BYTES);
                 } else {
                     stage_bytes = CG * Cfg::STAGE_BYTES;
                 }
@@ -1262,7 +1261,8 @@ void choose_plain_tiles(gpu_kernels::Nvfp4Params& p, const uint8_t* B, int force
         const float ns = estimate(t, waves);
         if (ns < best_ns) { best_ns = ns; best = &t; }
     }
-    if (forced == 1064) best = &PLAIN_TILES[3];
+    for (const PlainTile& t : PLAIN_TILES)
+        if (forced == t.cta_group * 1000 + t.tile_n) best = t.cta_group == p.cta_group && t.tile_n == p.tile_n ? nullptr : &t;
     if (!best) return;
     const int tiles_m = (p.M + 128 * best->cta_group - 1) / (128 * best->cta_group);
     p.plain_cta_group = best->cta_group;
@@ -1310,7 +1310,8 @@ void prepare_format(gpu_kernels::Nvfp4Params& p, const uint8_t* A, const uint8_t
 
     int force = env_int("NVFP4_B200_VARIANT", 0);              // 0 auto, 2256 / 1256 / 1128 / 1064 for experiments
     const bool own_tiles = force != 0 && force != 1064;        // 1064: the plan as usual, its plain launches on 64-wide tiles
-    const int plain = force;
+    // the same codes: the plan as usual, its plain launches on these tiles
+    const int plain = force == 1064 ? force : env_int("NVFP4_B200_PLAIN_TILE", 0);
     if (!own_tiles) force = 0;
     // M and N need not be whole tiles: the scale arrays end in whole 128-row atoms whatever the row count (rows
     // the tensor does not have read as zeros through the tensor maps), and the variant is chosen for the sizes

@@ -539,6 +539,32 @@ def test_plain_launch_on_other_tiles(g, m, n, k, variant):
     plan.close()
 
 
+@pytest.mark.parametrize("m", [1, 8, 100, 120, 121, 128, 129, 300])
+@pytest.mark.parametrize("tile,n,k", [(2256, 1000, 1088), (2256, 72, 320), (1256, 1000, 1088), (1128, 328, 4160)])
+def test_plain_launch_on_every_kind_of_tile(g, m, tile, n, k, monkeypatch):
+    # a box of A is as tall as a short tensor, and of a CTA pair's tile either half may lie wholly beyond M or N: what a
+    # stage's barrier expects has to follow (the rule takes pairs for none of the shorter ones, so they are forced)
+    pa, sa = g.quantize(random_operand(m, k, seed=m + n))
+    pb, sb = g.quantize(random_operand(n, k, seed=m + k, scale=0.05))
+    monkeypatch.setenv("NVFP4_B200_PLAIN_TILE", str(tile))
+    plan = g.Nvfp4Gemm(pa, pb, sa, sb)
+    info = plan.info()
+    assert info["launch_cta_group"] * 1000 + info["launch_tile_n"] == tile, info
+    whole = torch.full((m + 3, n), float("nan"), dtype=torch.float16, device="cuda")
+    whole[m:] = 77.0
+    out = plan.run(whole[:m])
+    plan.validate()
+    assert_gemm_close(out, to_np(g.dequantize(pa, sa) @ g.dequantize(pb, sb).T), f"tile {tile} {m}x{n}x{k}")
+    assert bool((whole[m:] == 77.0).all()), "rows beyond M were written"
+    for mode in (1, 2):                                      # the halves of a ring fill that wait for the launch in front
+        plan.set_option("static_operands", mode)
+        outs = [plan.run(nan_output(m, n)) for _ in range(3)]
+        torch.cuda.synchronize()
+        assert all(torch.equal(o, out) for o in outs)
+    plan.validate()
+    plan.close()
+
+
 @pytest.mark.parametrize("m,n,k", [(128, 256, 2048), (256, 512, 256), (384, 640, 512)])
 def test_output_that_starts_on_a_16_byte_boundary(g, m, n, k):
     # whole tiles into a C that is 16- but not 32-byte aligned: the same bits as into an aligned one
