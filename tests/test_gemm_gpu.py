@@ -53,9 +53,9 @@ def test_golden_cfg0(g, golden):
     # FP16 rounding of nearly equal FP32 sums: the two outputs may differ by one FP16 step on a few elements
     same = (out.cpu() == ref16).float().mean()
     assert same > 0.99, f"only {same:.4f} of FP16 outputs identical to the reference's"
-    for variant in (1256, 1128):
+    for variant in (2256, 1256, 1128):
         out_v, info_v = run_plan(g, pa, sa, pb, sb, variant=variant)
-        assert info_v["cta_group"] == 1
+        assert info_v["launch_cta_group"] * 1000 + info_v["launch_tile_n"] == variant, info_v
         assert_gemm_close(out_v, f["c_f32"], f"cfg0 variant {variant}")
 
 
@@ -71,6 +71,8 @@ SHAPES = [
     (1024, 1024, 1536, 1256),
     (1024, 1024, 1536, 1128),
     (4096, 2048, 256, None),        # many tiles, single K step: epilogue-bound
+    (2048, 4096, 2048, 2256),       # the instance of the large products: whole 256 x 256 tiles on CTA pairs
+    (512, 768, 512, 2256),
 ]
 
 
@@ -80,7 +82,8 @@ def test_shapes_against_oracle(g, m, n, k, variant):
     b = random_operand(n, k, seed=2 + m + n + k, scale=0.02)
     pa, sa = g.quantize(a)
     pb, sb = g.quantize(b)
-    out, _ = run_plan(g, pa, sa, pb, sb, variant=variant)
+    out, info = run_plan(g, pa, sa, pb, sb, variant=variant)
+    assert variant is None or info["launch_cta_group"] * 1000 + info["launch_tile_n"] == variant, info
     ref = O.gemm_f32(to_np(pa), to_np(sa), to_np(pb), to_np(sb))
     assert_gemm_close(out, ref, f"{m}x{n}x{k}")
 
@@ -94,6 +97,8 @@ K_TAIL_SHAPES = [
     (2048, 1024, 2240, None),       # ring wraps with a partial last step, K walks that start anywhere
     (512, 512, 1472, 1256),
     (512, 512, 1472, 1128),
+    (256, 256, 320, 2256),
+    (2048, 1024, 2240, 2256),
 ]
 
 
@@ -317,7 +322,7 @@ def test_distinct_scale_everywhere(g):
     sb_raw = (36 + (np.arange(n)[:, None] * 5 + np.arange(k // 16)[None, :] * 11) % 28).astype(np.uint8)
     sa, sb = O.pack_scales(sa_raw), O.pack_scales(sb_raw)
     ref = O.gemm_f32(pa, sa, pb, sb)
-    for variant in (None, 1256, 1128):
+    for variant in (None, 2256, 1256, 1128):
         out, _ = run_plan(g, *(torch.from_numpy(x).cuda() for x in (pa, sa, pb, sb)), variant=variant)
         assert_gemm_close(out, ref, f"distinct scales, variant {variant}")
 
@@ -468,8 +473,9 @@ EDGE_SHAPES = [
 ]
 
 
+@pytest.mark.parametrize("own_tiles", [False, True])
 @pytest.mark.parametrize("m,n,k,variant", EDGE_SHAPES)
-def test_m_and_n_that_are_not_whole_tiles(g, m, n, k, variant):
+def test_m_and_n_that_are_not_whole_tiles(g, m, n, k, variant, own_tiles, monkeypatch):
     a = random_operand(m, k, seed=m + 3 * k)
     b = random_operand(n, k, seed=n + 5 * k, scale=0.05)
     pa, sa = g.quantize(a)
@@ -479,9 +485,12 @@ def test_m_and_n_that_are_not_whole_tiles(g, m, n, k, variant):
     ua = g.unpack_scales(sa, -(-m // 128) * 128, k); ua[m:] = 0x7F
     ub = g.unpack_scales(sb, -(-n // 128) * 128, k); ub[n:] = 0x7F
     sa2, sb2 = g.pack_scales(ua), g.pack_scales(ub)
+    if own_tiles:                                            # the rule takes narrower ones for most of these
+        monkeypatch.setenv("NVFP4_B200_PLAIN_TILE", str(variant))
     plan = g.Nvfp4Gemm(pa, pb, sa2, sb2)
     info = plan.info()
     assert info["cta_group"] * 1000 + info["tile_n"] == variant, info
+    assert not own_tiles or info["launch_cta_group"] * 1000 + info["launch_tile_n"] == variant, info
     whole = torch.full((m + 3, n), float("nan"), dtype=torch.float16, device="cuda")
     whole[m:] = 77.0
     out = whole[:m]
@@ -533,9 +542,41 @@ def test_plain_launch_on_other_tiles(g, m, n, k, variant):
     ref = g.dequantize(pa, sa) @ g.dequantize(pb, sb).T
     assert_gemm_close(out, to_np(ref), f"plain tiles {m}x{n}x{k}")
     assert bool((whole[m:] == 77.0).all()), "rows beyond M were written"
-    # the plan's own tiles take every sum in the same order: the same bits
     own, _ = run_plan(g, pa, sa2, pb, sb2, variant=info["cta_group"] * 1000 + info["tile_n"])
-    assert torch.equal(out, own)
+    if info["launch_issuers"] == 1:                          # the plan's own tiles take every sum in the same order: the same bits
+        assert torch.equal(out, own)
+    else:
+        assert_within_summation_order(g, (out, own), pa, sa, pb, sb)
+    plan.close()
+
+
+def assert_within_summation_order(g, outs, pa, sa, pb, sb):
+    """Each of `outs` against the exact product: one rounding to FP16 (2^-11 of the value, half a subnormal step), and in
+    FP32 no more than an error of 2^-22 of the sum of the magnitudes (two units in the last place, so that a truncating
+    adder passes too) for each of the K / 64 MMAs and the addition of two accumulators."""
+    a, b = g.dequantize(pa, sa).double(), g.dequantize(pb, sb).double()
+    exact, magnitude = a @ b.T, a.abs() @ b.abs().T
+    bound = exact.abs() * 2.0 ** -11 + 2.0 ** -25 + magnitude * ((a.shape[1] // 64 + 1) * 2.0 ** -22)
+    for out in outs:
+        assert not torch.isnan(out).any()
+        assert bool(((out.double() - exact).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("m,n,k", [(5, 520, 4096), (128, 1536, 8192), (64, 2048, 4160)])
+def test_two_issuers_on_operands_of_wide_range(g, m, n, k):
+    # even and odd ring steps are summed apart there: block scales over 2^10, so that FP32 sums depend on their order
+    a = random_operand(m, k, seed=m, dtype=torch.float32)
+    spread = torch.rand((m, k // 16), generator=torch.Generator(device="cuda").manual_seed(k), device="cuda") - 0.5
+    pa, sa = g.quantize((a * torch.exp2(10 * spread).repeat_interleave(16, 1)).bfloat16())
+    pb, sb = g.quantize(random_operand(n, k, seed=n, scale=0.02))
+    plan = g.Nvfp4Gemm(pa, pb, sa, sb)
+    info = plan.info()
+    assert info["launch_issuers"] == 2, info
+    out = plan.run(nan_output(m, n))
+    plan.validate()
+    own, own_info = run_plan(g, pa, sa, pb, sb, variant=info["cta_group"] * 1000 + info["tile_n"])
+    assert own_info["launch_issuers"] == 1
+    assert_within_summation_order(g, (out, own), pa, sa, pb, sb)
     plan.close()
 
 
@@ -622,7 +663,7 @@ def test_full_size_square(g, size):
     pb, sb = g.quantize(b)
     del a, b
     out, info = run_plan(g, pa, sa, pb, sb)
-    assert info["cta_group"] == 2
+    assert info["launch_cta_group"] == 2 and info["launch_tile_n"] == 256
     ref = fp32_reference_on_gpu(g, pa, sa, pb, sb)
     assert_gemm_close(out, ref, f"{size}^3 vs FP32 dequantise-then-matmul")
     if size == 8192:
@@ -638,7 +679,7 @@ def test_full_size_skinny(g):
     pa, sa = g.quantize(random_operand(m, k, seed=0))
     pb, sb = g.quantize(random_operand(n, k, seed=1, scale=0.02))
     out, info = run_plan(g, pa, sa, pb, sb)
-    assert info["cta_group"] == 1
+    assert info["launch_cta_group"] == 1 and info["launch_tile_n"] == 256
     assert_gemm_close(out, fp32_reference_on_gpu(g, pa, sa, pb, sb), "skinny vs FP32 dequantise-then-matmul")
 
 
