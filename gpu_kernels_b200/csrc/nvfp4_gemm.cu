@@ -1731,15 +1731,17 @@ void grouped_launch_fused(const GroupedGemm& p, void* C, int out_bf16, uint8_t* 
     g.slot_rows = slot_rows;
     const int dev = p.device, units = p.units;
     const bool pdl = env_int("NVFP4_B200_PDL", 1) != 0;
+    // as for a dense C: 16-byte stores where C itself does not start on a 32-byte boundary
+    const bool masked = p.block_valid || !g.c_rows_32;
     if (p.block_rows == 256) {
         if (fused) launch_instance<2, 256, EPI_ACT>(dev, units, p.A, p.B, p.SFA, p.SFB, tmC, g, stream, pdl);
         else if (row_dst) launch_instance<2, 256, EPI_SCATTER_ROWS>(dev, units, p.A, p.B, p.SFA, p.SFB, tmC, g, stream, pdl);
-        else if (p.block_valid) launch_instance<2, 256, EPI_DIRECT_EDGE>(dev, units, p.A, p.B, p.SFA, p.SFB, tmC, g, stream, pdl);
+        else if (masked) launch_instance<2, 256, EPI_DIRECT_EDGE>(dev, units, p.A, p.B, p.SFA, p.SFB, tmC, g, stream, pdl);
         else launch_instance<2, 256, EPI_DIRECT>(dev, units, p.A, p.B, p.SFA, p.SFB, tmC, g, stream, pdl);
     } else {
         if (fused) launch_instance<1, 256, EPI_ACT>(dev, units, p.A, p.B, p.SFA, p.SFB, tmC, g, stream, pdl);
         else if (row_dst) launch_instance<1, 256, EPI_SCATTER>(dev, units, p.A, p.B, p.SFA, p.SFB, tmC, g, stream, pdl);
-        else if (p.block_valid) launch_instance<1, 256, EPI_DIRECT_EDGE>(dev, units, p.A, p.B, p.SFA, p.SFB, tmC, g, stream, pdl);
+        else if (masked) launch_instance<1, 256, EPI_DIRECT_EDGE>(dev, units, p.A, p.B, p.SFA, p.SFB, tmC, g, stream, pdl);
         else launch_instance<1, 256, EPI_DIRECT>(dev, units, p.A, p.B, p.SFA, p.SFB, tmC, g, stream, pdl);
     }
 }

@@ -389,6 +389,16 @@ def test_plain_second_gemm_writes_only_the_real_rows(g, block_rows):
     everything, masked = outs
     assert torch.equal(masked[real], everything[real])
     assert bool((masked[~real] == -3.0).all()) and not bool((everything[~real] == -3.0).all())
+    # a C that starts on a 16-byte boundary, not on a 32-byte one: 16-byte stores, the same bits, nothing around it written
+    flat = torch.full((layer.out_pool.numel() + 16,), 77.0, dtype=torch.bfloat16, device="cuda")
+    shifted = flat[8:8 + layer.out_pool.numel()].view_as(layer.out_pool)
+    assert shifted.data_ptr() % 32 == 16
+    for table, want in ((None, everything), (layer.block_valid.data_ptr(), masked)):
+        _lib.check(lib.gpu_kernels_nvfp4_grouped_set_valid_rows(fc2, table))
+        shifted.fill_(-3.0)
+        _lib.check(lib.gpu_kernels_nvfp4_grouped_run(fc2, shifted.data_ptr(), 1, stream))
+        torch.cuda.synchronize()
+        assert torch.equal(shifted[:rows], want) and bool((flat[:8] == 77.0).all()) and bool((flat[-8:] == 77.0).all())
     assert lib.gpu_kernels_nvfp4_validate(None) == 0
     layer.close()
 
