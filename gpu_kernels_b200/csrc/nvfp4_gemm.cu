@@ -1354,6 +1354,8 @@ void prepare(gpu_kernels::Nvfp4Params& p, const uint8_t* A, const uint8_t* B, co
     prepare_format(p, A, B, SFA, SFB, M, N, K, false);
 }
 
+int rows_start_on_32(const void* c, int ldc) { return (reinterpret_cast<uintptr_t>(c) & 31) == 0 && ldc % 16 == 0; }
+
 // table: device memory of gather_table_bytes(world), filled here (on `stream`) with one tensor map and one
 // base pointer per destination; buffers: host array of `world` device pointers to the full [M, n_total] C.
 size_t gather_table_bytes(int world) { return size_t(world) * (sizeof(CUtensorMap) + sizeof(void*)); }
@@ -1379,6 +1381,8 @@ void set_gather(gpu_kernels::Nvfp4Params& p, void* const* buffers, int world, in
     p.gather_world = world;
     p.gather_col0 = col0;
     p.gather_ldc = n_total;
+    p.gather_rows_32 = n_total % 16 == 0;
+    for (int r = 0; r < world; ++r) p.gather_rows_32 &= rows_start_on_32(buffers[r], n_total);
     p.gather_maps = table;
     p.gather_ptrs = static_cast<uint8_t*>(table) + size_t(world) * sizeof(CUtensorMap);
 }
@@ -1422,8 +1426,6 @@ void enable_split_k(gpu_kernels::Nvfp4Params& p, void* workspace, size_t bytes, 
     p.route = nullptr;                                                   // slices are dealt in item order
     p.clusters = (p.M / (128 * p.cta_group)) * (p.N / p.tile_n) * s;     // one (tile, slice) per unit
 }
-
-int rows_start_on_32(const void* c, int ldc) { return (reinterpret_cast<uintptr_t>(c) & 31) == 0 && ldc % 16 == 0; }
 
 GemmArgs dense_args(const gpu_kernels::Nvfp4Params& p, void* c, unsigned long long* prof) {
     const int tile_m = 128 * p.cta_group;
@@ -1545,7 +1547,11 @@ void launch_plain(const gpu_kernels::Nvfp4Params& p, const CUtensorMap& tmC, con
 void launch_with(const gpu_kernels::Nvfp4Params& p, void* C, cudaStream_t stream, unsigned long long* prof) {
     if (!C || (reinterpret_cast<uintptr_t>(C) & 15)) throw std::invalid_argument("nvfp4 gemm: C must be 16-byte aligned");
     if (prof && (p.split_k > 1 || p.gather_world)) throw std::invalid_argument("nvfp4 gemm profile: plain plans only");
-    if ((reinterpret_cast<uintptr_t>(C) & 31) && (p.split_k > 1 || (prof && p.direct_store)))
+    // CTA pairs send the slab by TMA stores, which take 16-byte boundaries
+    if (p.gather_world && !p.gather_rows_32 && (p.cta_group == 1 || p.split_k > 1))
+        throw std::invalid_argument("nvfp4 gemm gather: this plan stores 32 bytes at a time: the full C buffers must be 32-byte "
+                                    "aligned and their width a multiple of 16");
+    if ((reinterpret_cast<uintptr_t>(C) & 31) && !p.gather_world && (p.split_k > 1 || (prof && p.direct_store)))
         throw std::invalid_argument("nvfp4 gemm: split-K and profiled launches store 32 bytes at a time: C must be 32-byte aligned");
     // only the staged route stores C through a map
     const CUtensorMap tmC = p.direct_store ? CUtensorMap{} : output_map(C, p.M, p.N, p.out_bf16 != 0);

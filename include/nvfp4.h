@@ -44,6 +44,7 @@ struct Nvfp4Params {
     void* split_k_workspace;        // flags + FP32 partial tiles, owned by the caller
     int gather_world;               // > 0: C goes to this many full-width buffers instead (see nvfp4_set_gather)
     int gather_col0, gather_ldc;
+    int gather_rows_32;             // 1: every row of every full C starts on a 32-byte boundary
     const void* gather_maps;
     const void* gather_ptrs;
     int out_bf16;                   // 1: launch() writes bfloat16 instead of FP16 through the same pointer

@@ -127,8 +127,9 @@ int gpu_kernels_nvfp4_plan_set_option(void* plan, const char* key, int value);
  * from its epilogue into ALL `world` buffers (host array of device pointers: this rank's full C and the
  * peers', opened with gpu_kernels_nvfp4_ipc_open); nothing is written through C then (still a valid device
  * pointer of M * N elements, e.g. this rank's buffer). The caller puts a
- * barrier between the ranks before reading, and before the next launch overwrites. world = 0 switches it
- * off. Not inside stream capture (synchronises once). */
+ * barrier between the ranks before reading, and before the next launch overwrites. The buffers are 16-byte aligned and
+ * n_total a multiple of 8; 32-byte aligned and a multiple of 16 for plans on single CTAs or with split_k (their launch
+ * refuses others). world = 0 switches it off. Not inside stream capture (synchronises once). */
 int gpu_kernels_nvfp4_plan_set_gather(void* plan, void* const* buffers, int world, int col0, int n_total);
 /* Fills info[0..15] = {M, N, K, units, cta_group, tile_n, group_m, stages, split_k, k_skew, direct_store,
  * out_bf16, l2_side order in use, clusters on L2 side 0, on side 1, ragged tiles (0 = uniform tiling)}: the plan's own

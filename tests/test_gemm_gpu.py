@@ -649,6 +649,34 @@ def test_mxfp4_narrow_tiles(g, m, n, k):
     plan.close()
 
 
+@pytest.mark.parametrize("m,n,k,split_k,n_total,offset,served", [
+    (128, 512, 1024, False, 528, 0, True), (128, 512, 1024, False, 520, 0, False), (128, 512, 1024, False, 528, 8, False),
+    (256, 512, 512, False, 520, 8, True),                     # CTA pairs: TMA stores
+    (128, 512, 4096, True, 512, 0, True), (128, 512, 4096, True, 520, 0, False),
+])
+def test_gather_into_rows_that_start_on_16_byte_boundaries(g, m, n, k, split_k, n_total, offset, served):
+    # one rank: the slab into a wider full C; register stores write 32 bytes at a time, and are refused where they cannot
+    import ctypes
+    from gpu_kernels_b200 import _lib
+    pa, sa = g.quantize(random_operand(m, k, seed=m + k))
+    pb, sb = g.quantize(random_operand(n, k, seed=n + k, scale=0.05))
+    plan = g.Nvfp4Gemm(pa, pb, sa, sb)
+    if split_k:
+        plan.set_option("split_k", 1)
+    flat = torch.full((m * n_total + 16,), 77.0, dtype=torch.float16, device="cuda")
+    full = flat[offset:offset + m * n_total].view(m, n_total)
+    _lib.check(_lib.load().gpu_kernels_nvfp4_plan_set_gather(plan._plan, (ctypes.c_void_p * 1)(full.data_ptr()), 1, 0, n_total))
+    if served:
+        plan.run(nan_output(m, n))
+        plan.validate()
+        assert_gemm_close(full[:, :n], to_np(g.dequantize(pa, sa) @ g.dequantize(pb, sb).T), f"gather {m}x{n}x{k}")
+        assert bool((full[:, n:] == 77.0).all())
+    else:
+        with pytest.raises(RuntimeError, match="32"):
+            plan.run(nan_output(m, n))
+    plan.close()
+
+
 def fp32_reference_on_gpu(g, pa, sa, pb, sb):
     """The reference's check (dequantise both operands, FP32 matmul) at full size on the GPU.
     The dequantise kernel is itself pinned bit-exactly to the oracle in test_quantize_gpu.py."""
