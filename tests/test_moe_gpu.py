@@ -398,7 +398,8 @@ def test_plain_second_gemm_writes_only_the_real_rows(g, block_rows):
         shifted.fill_(-3.0)
         _lib.check(lib.gpu_kernels_nvfp4_grouped_run(fc2, shifted.data_ptr(), 1, stream))
         torch.cuda.synchronize()
-        assert torch.equal(shifted[:rows], want) and bool((flat[:8] == 77.0).all()) and bool((flat[-8:] == 77.0).all())
+        assert torch.equal(shifted[:rows][real], want[real]) and bool((flat[:8] == 77.0).all()) and bool((flat[-8:] == 77.0).all())
+        assert bool((shifted[:rows][~real] == -3.0).all()) == (table is not None)      # padding rows: anything, or untouched
     assert lib.gpu_kernels_nvfp4_validate(None) == 0
     layer.close()
 
