@@ -18,7 +18,7 @@ Unless `--only` is given, the same invocation also measures the other configurat
 (16384^3, the skinny decode shape, the stand-alone quantiser, the expert layer at 1/64/1024/4096 tokens per
 GPU) with a shorter warm-up, and reports them under `configs`. After timing, results are checked (`parity`):
 sampled rows against the FP32 dequantise-then-matmul path and the CPU oracle, the fused all-gather against
-the NCCL route bit for bit, the expert layer on sampled tokens against the oracle; the ranks agree on the
+the NCCL route (bit for bit where both sum in one order), the expert layer on sampled tokens against the oracle; the ranks agree on the
 verdict through an all-reduce, and a failed check makes every rank exit non-zero.
 
 `--impl reference` times the reference's CPU path (dequantise both operands, FP32 matmul, FP16 rounding:
@@ -508,7 +508,7 @@ def run_gemm(args, ranks: Ranks, workload, sampler, main, gathers=("none",)):
     if info.get("l2_side"):
         result["placement_misses"] = plans[0].placement_misses()
     alg_bytes = algorithmic_bytes(m, n_local, k)
-    kernel = f"nvfp4_gemm_kernel<{info['cta_group']},{info['tile_n']}>"
+    kernel = f"nvfp4_gemm_kernel<{info['launch_cta_group']},{info['launch_tile_n']}>"
     result["roofline"] = tensor_roofline(flops / world, alg_bytes, ms, peaks, True, kernel,
                                          NCU_DRAM_BYTES_PER_LAUNCH.get(workload) if world == 1 else None)
 
@@ -535,7 +535,8 @@ def run_gemm(args, ranks: Ranks, workload, sampler, main, gathers=("none",)):
     ok, details = check_gemm(g, out, pa, sa, pb, sb, k, rank)
     parity = {"gemm_rank0_details": details}
 
-    # N > 1: the full C on every rank, fused into the epilogue or by NCCL; both timed, and compared bit for bit
+    # N > 1: the full C on every rank, fused into the epilogue or by NCCL; both timed, and compared: bit for bit, or to
+    # the last place where the NCCL route's plain launch has two issuers (even and odd K steps summed apart)
     gather_results = {}
     fulls = {}
     for mode in gathers:
@@ -573,6 +574,10 @@ def run_gemm(args, ranks: Ranks, workload, sampler, main, gathers=("none",)):
     if "fused" in fulls and "nccl" in fulls:
         same = bool(torch.equal(fulls["fused"], fulls["nccl"]))
         parity["fused_gather_equals_nccl_gather_bitwise"] = same
+        if not same and info["launch_issuers"] == 2:
+            apart = (fulls["fused"].double() - fulls["nccl"].double()).norm() / fulls["nccl"].double().norm()
+            parity["fused_gather_against_nccl_gather_rel"] = float(apart)
+            same = float(apart) <= 1e-4
         ok &= same
         mine = bool(torch.equal(fulls["nccl"][:, lo:hi], out))
         parity["gathered_slab_equals_local_slab"] = mine
@@ -1021,7 +1026,7 @@ def main():
     ap.add_argument("--gather", default="auto", choices=["auto", "none", "fused", "nccl"],
                     help="N>1, GEMM workloads: also time the step that leaves the full C on every rank: 'fused' = the GEMM's "
                          "epilogue stores the slab into all ranks' buffers over NVLink + a barrier kernel; 'nccl' = all-gather "
-                         "+ strided copy; auto = both (and compared bit for bit)")
+                         "+ strided copy; auto = both (and compared)")
     ap.add_argument("--l2-side", default="auto", choices=["auto", "on", "off"],
                     help="tile order of the dense GEMM: the plan's default, or force the L2-side-aware order on / off")
     ap.add_argument("--no-cpu", action="store_true", help="skip the CPU baseline leg")
