@@ -405,7 +405,7 @@ struct Roles {
             }
             // whole tiles may start anywhere in K and wrap; slices of a tile are walked in order
             // (see GemmArgs::k_skew); a dense C's walk depends on the 256 x 256 block of C, not on the tile, so that
-            // its sums are taken in the same order whatever the tiles are
+            // its sums are taken in the same order whatever the tiles are (but twins add even and odd steps apart)
             const uint32_t place = g.block_expert || Cfg::RAGGED ? t : uint32_t(tn * UN / 256 + 5 * (tm * Cfg::TILE_M / 256));
             const int k_first = (g.k_skew && g.split_k <= 1) ? int((place * uint32_t(g.k_skew)) % uint32_t(ksteps)) : 0;
             for (int step = seg.k0; step < seg.k1; ++step) {
@@ -655,7 +655,8 @@ struct Roles {
     // the first cols_left (a multiple of 8: N is) are written: in 32-byte stores where every row of C starts on a
     // 32-byte boundary (cols_left is then a multiple of 16), else in 16-byte ones, which write every sector of C in
     // two halves (the linear call 1000 x 8192 x 8192 47.5 us with 16-byte stores, 45.4 with 32-byte ones; the expert
-    // layer at 4096 tokens, whose second product takes this route, 826 and 770).
+    // layer, whose second product takes this route, 769 and 741 at 4096 tokens, 638 and 633 at 1024, medians of eight
+    // fresh layers each). With or without the evict-first hint the expert layer takes the same time.
     __device__ __forceinline__ void store_row_chunk_edge(uint16_t* dst, const uint32_t (&v)[EPI_COLS], float alpha, bool row_ok,
                                                          int cols_left) const {
         if (g.c_rows_32) {

@@ -225,8 +225,9 @@ class Nvfp4MoE:
         lib, s = _lib.load(), _lib.stream()
         routes = tokens * self.topk
         if self.world == 1 and routes <= 32768:
-            # one launch: histogram of the routes (by the plan's single CTA: 24576 routes take it less time than
-            # clearing, counting and copying as launches of their own), plan, arrival counters cleared
+            # One launch: histogram of the routes (by the plan's single CTA), plan, arrival counters cleared. Against
+            # clearing, counting and copying as launches of their own: 5 us of host time instead of 20; on the device
+            # 4.4 / 7.4 us at 1020 routes, 6.6 / 7.6 at 12288, 8.8 / 7.9 at 24576 (all on one expert 10.2 / 9.1).
             _lib.check(lib.gpu_kernels_nvfp4_moe_route_plan(
                 ids.data_ptr(), routes, self.counts_matrix.data_ptr(), self.experts, self.pool_rows, block_rows,
                 self.send_offset.data_ptr(), self.seg_src.data_ptr(), self.seg_pool.data_ptr(),

@@ -39,7 +39,8 @@ struct Nvfp4Params {
     int device;                     // device the plan was prepared on
     int c_evict_first;              // 1: C is stored with the evict-first L2 policy
     int direct_store;               // 1: epilogue writes C from registers instead of TMA stores
-    int k_skew;                     // tile t starts its K walk at step (t * k_skew) % steps and wraps; 0 = off
+    int k_skew;                     // a tile starts its K walk at step (place * k_skew) % steps and wraps, place counting
+                                    // the 256-wide blocks of C (ragged tiles: the tile's index); 0 = off
     int split_k;                    // S > 1: S units per tile, each with 1/S of the K steps (see below)
     void* split_k_workspace;        // flags + FP32 partial tiles, owned by the caller
     int gather_world;               // > 0: C goes to this many full-width buffers instead (see nvfp4_set_gather)

@@ -97,7 +97,7 @@ int gpu_kernels_nvfp4_linear(void* plan, const void* x, int dtype, void* C, void
 /* FP32 global scale: C = fp16(alpha * accumulator). The reference fixes alpha = 1 (nvfp4_bridge.cu:101). */
 int gpu_kernels_nvfp4_plan_set_alpha(void* plan, float alpha);
 /* Tuning knobs. key: "group_m" (tile rows per rasterisation band, >= 1); "c_evict_first" (0/1: L2 policy
- * of the C stores); "direct_store" (0/1: epilogue writes C from registers instead of staging it for TMA stores);
+ * of the staged route's TMA stores of C; register stores of 32 bytes always carry it); "direct_store" (0/1: epilogue writes C from registers instead of staging it for TMA stores);
  * "ragged_tiles" (T: deal the columns of a plan with M = 128, in units of 64, to T single-CTA tiles of two widths
  * (2/3 or 3/4 units) instead of N/256 tiles of 256 columns, e.g. T = the SM count where N/256 tiles would leave SMs idle; 0 = uniform
  * tiles, the default);
@@ -114,7 +114,8 @@ int gpu_kernels_nvfp4_plan_set_alpha(void* plan, float alpha);
  * the side of the L2 they sit on and deals each side one contiguous part of the tile sequence; fails when the
  * plan's grid does not fill the GPU or the census finds no two sides; results never depend on it; not inside
  * stream capture);
- * "k_skew" (>= 0: tile t starts its K walk at step (t * k_skew) % steps; 0 = every tile at K = 0);
+ * "k_skew" (>= 0: a tile starts its K walk at step (place * k_skew) % steps, place counting the 256-wide blocks of C,
+ * column + 5 * row, or the index of a ragged tile; 0 = every tile at K = 0);
  * "split_k" (0/1, default 0: four units per tile, each with a quarter of the K steps, partial sums combined
  * through a workspace the plan allocates. Offered for shapes with at most a quarter as many tiles as SMs and
  * at least 16 K steps of 256 (10-13 % faster there); refused for others. The units of such a launch wait
