@@ -1220,6 +1220,8 @@ std::atomic<unsigned> g_next_slot{0};
 // GemmArgs::a_box_rows). With whole boxes 8 x 8192 x 8192 on 128-wide tiles took 20.3 us, with 8-row boxes 14.8 us.
 int a_box_rows(int M) { return M < BLOCK_M ? (M + 7) / 8 * 8 : BLOCK_M; }
 
+constexpr int AUTO_GROUP_M = -(1 << 30);          // NVFP4_B200_GROUP_M is not set: band_rows
+
 // About sqrt(units) tile rows per band keeps the A and B panels of the tiles in flight balanced.
 // Measured at 16384^3 (64 x 64 tiles, operands beyond L2): bands of 16 beat 8 by 1.3 %, 32 and 4 lose 10 %;
 // at 8192^3 (everything L2-resident) the band height does not matter.
@@ -1244,7 +1246,7 @@ int band_rows(int units, int tiles_m) {
 struct PlainTile { int cta_group, tile_n; float step_ns, tail_ns; };
 constexpr PlainTile PLAIN_TILES[] = {{2, 256, 380.0f, 1000.0f}, {1, 256, 430.0f, 1000.0f}, {1, 128, 320.0f, 500.0f}, {1, 64, 290.0f, 300.0f}};
 
-void choose_plain_tiles(gpu_kernels::Nvfp4Params& p, const uint8_t* B, int forced) {
+void choose_plain_tiles(gpu_kernels::Nvfp4Params& p, const uint8_t* B, int forced, int group_m) {
     const int steps = (p.K + STAGE_K - 1) / STAGE_K;
     const float hbm_ns = float(p.N) * float(p.K) * (p.mx ? 0.53125f : 0.5625f) / 6500.0f;
     auto tiles = [&](const PlainTile& t) { return ((p.M + 128 * t.cta_group - 1) / (128 * t.cta_group)) * ((p.N + t.tile_n - 1) / t.tile_n); };
@@ -1269,7 +1271,7 @@ void choose_plain_tiles(gpu_kernels::Nvfp4Params& p, const uint8_t* B, int force
     p.plain_cta_group = best->cta_group;
     p.plain_tile_n = best->tile_n;
     p.plain_units = std::min(fit_units(p.device, best->cta_group, best->tile_n), tiles(*best));
-    p.plain_group_m = std::max(1, std::min(env_int("NVFP4_B200_GROUP_M", band_rows(p.plain_units, tiles_m)), tiles_m));
+    p.plain_group_m = std::max(1, std::min(group_m != AUTO_GROUP_M ? group_m : band_rows(p.plain_units, tiles_m), tiles_m));
     p.plain_B = operand_map(B, p.N, p.K, best->tile_n / best->cta_group);
 }
 
@@ -1309,10 +1311,11 @@ void prepare_format(gpu_kernels::Nvfp4Params& p, const uint8_t* A, const uint8_t
     p.device = device;
     p.c_evict_first = env_int("NVFP4_B200_C_EVICT_FIRST", 1);
 
-    int force = env_int("NVFP4_B200_VARIANT", 0);              // 0 auto, 2256 / 1256 / 1128 / 1064 for experiments
-    const bool own_tiles = force != 0 && force != 1064;        // 1064: the plan as usual, its plain launches on 64-wide tiles
-    // the same codes: the plan as usual, its plain launches on these tiles
-    const int plain = force == 1064 ? force : env_int("NVFP4_B200_PLAIN_TILE", 0);
+    // 0 auto; for experiments 2256 / 1256 / 1128: the plan on these tiles; 1064, or 10000 + any of the four: the plan as
+    // usual, its plain launches on these tiles. (One variable: every look-up costs a plan 0.1 us.)
+    int force = env_int("NVFP4_B200_VARIANT", 0);
+    const int plain = force == 1064 ? force : force > 10000 ? force - 10000 : 0;
+    const bool own_tiles = force != 0 && plain == 0;
     if (!own_tiles) force = 0;
     // M and N need not be whole tiles: the scale arrays end in whole 128-row atoms whatever the row count (rows
     // the tensor does not have read as zeros through the tensor maps), and the variant is chosen for the sizes
@@ -1335,7 +1338,8 @@ void prepare_format(gpu_kernels::Nvfp4Params& p, const uint8_t* A, const uint8_t
     const int tiles = (Mp / (128 * p.cta_group)) * (Np / p.tile_n);
     p.clusters = std::min(fit_units(device, p.cta_group, p.tile_n), tiles);
     const int tiles_m = Mp / (128 * p.cta_group);
-    p.group_m = std::max(1, std::min(env_int("NVFP4_B200_GROUP_M", band_rows(p.clusters, tiles_m)), tiles_m));
+    const int group_m = env_int("NVFP4_B200_GROUP_M", AUTO_GROUP_M);
+    p.group_m = std::max(1, std::min(group_m != AUTO_GROUP_M ? group_m : band_rows(p.clusters, tiles_m), tiles_m));
     // Measured: 128x28672x8192 30.2 -> 28.9 us, 8192^3 199.8 -> 199.0 us with the tiles' K walks de-phased.
     p.k_skew = env_int("NVFP4_B200_K_SKEW", 11);
     // One tile row whose 256-column tiles would leave SMs idle can deal its columns, in units of 64, to as many
@@ -1345,7 +1349,7 @@ void prepare_format(gpu_kernels::Nvfp4Params& p, const uint8_t* A, const uint8_t
     // launches: 28.5 against 24.7-26.1 us).
     if (!mx && env_int("NVFP4_B200_RAGGED", 0)) set_ragged_tiles(p, B, fit_units(device, 1, 256));
     p.pdl = env_int("NVFP4_B200_PDL", 1);
-    if (!own_tiles) choose_plain_tiles(p, B, plain);
+    if (!own_tiles) choose_plain_tiles(p, B, plain, group_m);
     p.status_slot = 1 + int(g_next_slot.fetch_add(1, std::memory_order_relaxed) % unsigned(STATUS_SLOTS - 1));
     (void)status_base(device);
 }

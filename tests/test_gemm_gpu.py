@@ -486,7 +486,7 @@ def test_m_and_n_that_are_not_whole_tiles(g, m, n, k, variant, own_tiles, monkey
     ub = g.unpack_scales(sb, -(-n // 128) * 128, k); ub[n:] = 0x7F
     sa2, sb2 = g.pack_scales(ua), g.pack_scales(ub)
     if own_tiles:                                            # the rule takes narrower ones for most of these
-        monkeypatch.setenv("NVFP4_B200_PLAIN_TILE", str(variant))
+        monkeypatch.setenv("NVFP4_B200_VARIANT", str(10000 + variant))
     plan = g.Nvfp4Gemm(pa, pb, sa2, sb2)
     info = plan.info()
     assert info["cta_group"] * 1000 + info["tile_n"] == variant, info
@@ -587,7 +587,7 @@ def test_plain_launch_on_every_kind_of_tile(g, m, tile, n, k, monkeypatch):
     # stage's barrier expects has to follow (the rule takes pairs for none of the shorter ones, so they are forced)
     pa, sa = g.quantize(random_operand(m, k, seed=m + n))
     pb, sb = g.quantize(random_operand(n, k, seed=m + k, scale=0.05))
-    monkeypatch.setenv("NVFP4_B200_PLAIN_TILE", str(tile))
+    monkeypatch.setenv("NVFP4_B200_VARIANT", str(10000 + tile))
     plan = g.Nvfp4Gemm(pa, pb, sa, sb)
     info = plan.info()
     assert info["launch_cta_group"] * 1000 + info["launch_tile_n"] == tile, info
